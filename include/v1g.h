@@ -453,8 +453,8 @@ int v1g_selftest_bounded_wait(V1GHandle* h, long long polls, void* stream);
  * kernel even where the register-resident one applies), "spin_limit" (iterations a grid-barrier
  * wait may spin before giving up), "no_meta" (1 = the rollout kernels read the plain post / sid /
  * weight arrays instead of the packed 8-byte synapse records), "no_q_pack" (1 = fp32 rows in the
- * backward ring for a batch of 5 instead of 24-bit floats), "pair_rows" (1 = two steps per 32-byte
- * row in the backward ring, halving the L2 requests of delays >= 2; measured slower, off by default), "phase_timers" (1 = per-block phase
+ * backward ring for a batch of 5 instead of 24-bit floats), "pair_rows" (accepted, without effect: a pass over
+ * the backward ring serves three steps anyway), "phase_timers" (1 = per-block phase
  * times, read with v1g_get_phase_times), "l2_window", "csr_evict_first" (cache-policy
  * experiments).  No counterpart in the reference. */
 int v1g_set_option(V1GHandle* h, const char* name, long long value);

@@ -24,7 +24,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
          "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC]
 # Gradient kernels are held to 1e-4, not to bit-equality, so they may contract multiply-adds; so
 # may the LGN filters, whose sums run in another order than the reference's convolutions anyway.
-FMAD_OK = {"v1g_rollout_bwd.cu", "v1g_lgn.cu"}
+FMAD_OK = ("v1g_rollout_bwd", "v1g_lgn.cu")
 
 
 def sources():
@@ -47,7 +47,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
     def compile_one(src):
         obj = os.path.join(out_dir, src[:-3] + ".o")
-        fmad = [] if src in FMAD_OK else ["-fmad=false"]
+        fmad = [] if src.startswith(FMAD_OK) else ["-fmad=false"]
         cmd = [NVCC, *FLAGS, *fmad, *extra, "-c", os.path.join(CSRC, src), "-o", obj]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:

@@ -112,11 +112,8 @@ static void free_source(V1GSource& s) {
   cudaFree(s.in_perm);
   cudaFree(s.w_in);
   cudaFree(s.w_ref);
-  for (int p = 0; p < 2; ++p) {
-    cudaFree(s.pair_ptr[p]);
-    cudaFree(s.pair_rec[p]);
-    cudaFree(s.pair_j[p]);
-  }
+  cudaFree(s.brow);
+  cudaFree(s.brec);
   s = V1GSource();
 }
 
@@ -282,11 +279,7 @@ extern "C" int v1g_set_connectivity(V1GHandle* h, int source, int64_t nnz,
   }
   s.post_sorted = sorted;
   s.in_ptr_host = in_ptr;
-  if (source == V1G_SRC_REC && want_syn8) {
-    s.rowptr_host = rowptr;
-    s.syn8x_host.resize((size_t)nnz);
-    for (int64_t i = 0; i < nnz; ++i) s.syn8x_host[(size_t)i] = syn8[(size_t)i].x;
-  }
+  if (source == V1G_SRC_REC && want_syn8) s.rowptr_host = rowptr;
   int rc;
   if ((rc = upload(h, &s.rowptr, rowptr.data(), rowptr.size()))) return rc;
   if ((rc = upload(h, &s.post, post.data(), post.size()))) return rc;
@@ -391,58 +384,58 @@ __global__ void permute_weights_kernel(const float* __restrict__ w_ref,
   for (; i < nnz; i += stride) w[i] = w_ref[perm[i]];
 }
 
-// weights into the gather-ordered record copies of the paired backward ring
-__global__ void pair_weights_kernel(const float* __restrict__ w, const int32_t* __restrict__ pos,
-                                    uint2* __restrict__ rec, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (; i < n; i += stride) rec[i].y = __float_as_uint(w[pos[i]]);
-}
-
-static void refresh_pair_weights(V1GSource& s, cudaStream_t st) {
-  if (!s.pair_built) return;
-  for (int p = 0; p < 2; ++p) {
-    if (s.pair_len[p] == 0) continue;
-    const int blocks = (int)std::min<int64_t>((s.pair_len[p] + 255) / 256, 148 * 16);
-    pair_weights_kernel<<<blocks, 256, 0, st>>>(s.w, s.pair_j[p], s.pair_rec[p], s.pair_len[p]);
-    v1g_count_launches(1);
-  }
-}
-
-int v1g_build_pair_tables(V1GHandle* h, cudaStream_t st) {
-  V1GSource& s = h->src[V1G_SRC_REC];
-  if (s.pair_built) return V1G_OK;
-  if (s.rowptr_host.empty() || !s.syn8)
-    return v1g_fail(h, V1G_ESTATE, "the paired backward ring needs the packed records of the recurrent source");
-  const int D = s.delays;
-  const int64_t n_src = s.n_src;
-  for (int p = 0; p < 2; ++p) {
-    std::vector<int32_t> ptr((size_t)n_src + 1), pos;
-    std::vector<uint2> rec;
-    pos.reserve((size_t)s.nnz);
-    for (int64_t n = 0; n < n_src; ++n) {
-      ptr[(size_t)n] = (int32_t)pos.size();
-      const int32_t* rp = s.rowptr_host.data() + n * D;
-      for (int j = rp[0]; j < rp[1]; ++j) pos.push_back(j);            // delay 1
-      for (int d = 1 + p; d < D; d += 2)                                // delays 2 + p, 4 + p, ...
-        for (int j = rp[d]; j < rp[d + 1]; ++j) pos.push_back(j);
+// Padded records of the backward gather, one warp per source neuron: the whole record, or its weight only.
+__global__ void __launch_bounds__(256) bwd_records_kernel(const int32_t* __restrict__ rowptr, int D, int64_t n_src,
+                                                          const int32_t* __restrict__ brow, const uint2* __restrict__ syn8,
+                                                          const float* __restrict__ w, int types, int weights_only,
+                                                          uint2* __restrict__ rec) {
+  const int lane = threadIdx.x & 31;
+  const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); n < n_src; n += stride) {
+    const int j0 = rowptr[n * D], len = rowptr[(n + 1) * D] - j0;
+    const int64_t o0 = (int64_t)brow[n] * V1G_ROW_PAD, o1 = (int64_t)brow[n + 1] * V1G_ROW_PAD;
+    for (int k = lane; k < (int)(o1 - o0); k += 32) {
+      if (weights_only) {
+        if (k < len) rec[o0 + k].y = __float_as_uint(w[j0 + k]);
+      } else {
+        // the padding repeats the row's last record with weight 0: its reads join those of the lane before
+        const int j = j0 + min(k, len - 1);
+        const unsigned x = syn8[j].x;
+        rec[o0 + k] = make_uint2(types <= 8 ? ((x & 0x3fffffu) * (unsigned)types + ((x >> 22) & 127u)) | (x & 0xe0000000u) : x,
+                                 k < len ? __float_as_uint(w[j]) : 0u);
+      }
     }
-    ptr[(size_t)n_src] = (int32_t)pos.size();
-    rec.resize(pos.size());
-    for (size_t i = 0; i < pos.size(); ++i) rec[i] = make_uint2(s.syn8x_host[(size_t)pos[i]], 0u);
-    s.pair_len[p] = (int64_t)pos.size();
-    int rc;
-    if ((rc = upload(h, &s.pair_ptr[p], ptr.data(), ptr.size()))) return rc;
-    if ((rc = upload(h, &s.pair_rec[p], rec.data(), rec.size()))) return rc;
-    if ((rc = upload(h, &s.pair_j[p], pos.data(), pos.size()))) return rc;
   }
-  s.pair_built = true;
-  refresh_pair_weights(s, st);
+}
+
+static void launch_bwd_records(const V1GHandle* h, V1GSource& s, int weights_only, cudaStream_t st) {
+  bwd_records_kernel<<<h->n_sms * 8, 256, 0, st>>>(s.rowptr, s.delays, s.n_src, s.brow, s.syn8, s.w, h->cfg.n_syn_types,
+                                                  weights_only, s.brec);
+  v1g_count_launches(1);
+}
+
+int v1g_build_bwd_records(V1GHandle* h, cudaStream_t st) {
+  V1GSource& s = h->src[V1G_SRC_REC];
+  if (s.brec) return V1G_OK;
+  std::vector<int32_t> brow((size_t)s.n_src + 1);
+  int64_t groups = 0;
+  for (int64_t n = 0; n < s.n_src; ++n) {
+    brow[(size_t)n] = (int32_t)groups;
+    groups += (s.rowptr_host[(size_t)(n + 1) * s.delays] - s.rowptr_host[(size_t)n * s.delays] + V1G_ROW_PAD - 1) / V1G_ROW_PAD;
+  }
+  brow[(size_t)s.n_src] = (int32_t)groups;
+  if ((groups + 16) * V1G_ROW_PAD > 0x7fffffffLL) return v1g_fail(h, V1G_ERANGE, "padded synapse records exceed 32-bit indexing");
+  int rc;
+  if ((rc = upload(h, &s.brow, brow.data(), brow.size()))) return rc;
+  // a pass may read (and ignore) records past the last row's end
+  V1G_CUDA(h, cudaMalloc((void**)&s.brec, (size_t)(groups + 16) * V1G_ROW_PAD * sizeof(uint2)));
+  V1G_CUDA(h, cudaMemsetAsync(s.brec + groups * V1G_ROW_PAD, 0, (size_t)16 * V1G_ROW_PAD * sizeof(uint2), st));
+  launch_bwd_records(h, s, 0, st);
   V1G_CUDA(h, cudaGetLastError());
   return V1G_OK;
 }
 
-// copy the weights into the packed synapse records of the backward gather
+// copy the weights into the packed synapse records of the forward scatter
 __global__ void syn8_weights_kernel(const float* __restrict__ w, uint2* __restrict__ syn8, int64_t nnz) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -470,7 +463,7 @@ extern "C" int v1g_set_weights(V1GHandle* h, int source, const float* w, void* s
     syn8_weights_kernel<<<blocks, threads, 0, st>>>(s.w, s.syn8, s.nnz);
     v1g_count_launches(1);
   }
-  refresh_pair_weights(s, st);
+  if (s.brec) launch_bwd_records(h, s, 1, st);
   if (!s.pos_set) {
     // the sign of each weight at construction is what SignedConstraint preserves (models.py:647-666)
     if (!s.pos_int) V1G_CUDA(h, cudaMalloc((void**)&s.pos_int, (size_t)s.nnz));
@@ -526,7 +519,7 @@ extern "C" int v1g_expadam_update_internal(V1GHandle* h, const float* grads_flat
         syn8_weights_kernel<<<blocks, 256, 0, st>>>(s.w, s.syn8, s.nnz);
         v1g_count_launches(1);
       }
-      refresh_pair_weights(s, st);
+      if (s.brec) launch_bwd_records(h, s, 1, st);
       if (src == V1G_SRC_BKG) {
         // the background weights also exist in caller's and CSR order (operator-level entry points)
         const int blocks = (int)std::min<int64_t>((s.nnz + 255) / 256, 148 * 16);
@@ -600,7 +593,7 @@ extern "C" int v1g_set_option(V1GHandle* h, const char* name, long long value) {
   } else if (!strcmp(name, "no_q_pack")) {
     h->opt_no_q_pack = value != 0;
   } else if (!strcmp(name, "pair_rows")) {
-    h->opt_pair_rows = value != 0;
+    // accepted and without effect: every pass over the backward ring serves three steps
   } else if (!strcmp(name, "l2_window")) {
     h->opt_l2_window = value != 0;
   } else if (!strcmp(name, "csr_evict_first")) {

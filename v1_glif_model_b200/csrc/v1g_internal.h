@@ -51,16 +51,13 @@ struct V1GSource {
   std::vector<int32_t> order_host;
   std::vector<int64_t> row_splits_host;
   std::vector<int32_t> in_ptr_host;  // host copy of in_ptr
-  // Recurrent source, built on first use of the paired backward ring: per delay parity p the records
-  // of every source neuron in gather order (its delay-1 bucket, then its buckets of delay d >= 2 with
-  // d - 1 = 1 + p, 3 + p, ...), the row starts and the CSR position of every entry.
-  std::vector<int32_t> rowptr_host;   // host copy of rowptr
-  std::vector<uint32_t> syn8x_host;   // host copy of the first word of syn8
-  int32_t* pair_ptr[2] = {nullptr, nullptr};  // [n_src + 1]
-  uint2* pair_rec[2] = {nullptr, nullptr};
-  int32_t* pair_j[2] = {nullptr, nullptr};
-  int64_t pair_len[2] = {0, 0};
-  bool pair_built = false;
+  // Recurrent source, built by the first backward rollout: the records as its gather walks them.  Every
+  // source neuron's row is padded with weight-0 records to a multiple of V1G_ROW_PAD, so that whole groups
+  // need no test for the row's end, and x holds the row of the ring directly: post * n_types + sid (up to 8
+  // synapse types; post | sid << 22 otherwise) | (delay-1) << 29.
+  std::vector<int32_t> rowptr_host;  // host copy of rowptr
+  int32_t* brow = nullptr;           // [n_src + 1] row starts in groups of V1G_ROW_PAD records
+  uint2* brec = nullptr;             // [brow[n_src] * V1G_ROW_PAD]
 };
 
 struct V1GHandle {
@@ -157,7 +154,6 @@ struct V1GHandle {
   int opt_force_smem_kernel = 0;  // never pick the register-resident forward kernel
   int opt_no_meta = 0;            // backward gather reads post / sid / w arrays instead of the packed records
   int opt_no_q_pack = 0;          // keep the backward Q rows in fp32 even for a batch of 5
-  int opt_pair_rows = 0;          // two steps per 32-byte row in the backward ring where the layout allows it
   int opt_l2_window = 0;          // pin the backward Q ring in L2 with an access-policy window
   int opt_csr_evict_first = 1;    // read the backward synapse stream with evict-first loads
   int opt_phase_timers = 0;   // record per-block phase times of the rollout kernels
@@ -177,8 +173,9 @@ void v1g_count_launches(int n);
 // message returned by v1g_last_error(NULL), for entry points that take no handle
 void v1g_set_global_error(const char* msg);
 
-// gather-ordered record tables of the recurrent source for the paired backward ring (built once)
-int v1g_build_pair_tables(V1GHandle* h, cudaStream_t st);
+// padded records of the recurrent source for the backward gather (built once, weights kept up to date)
+#define V1G_ROW_PAD 10
+int v1g_build_bwd_records(V1GHandle* h, cudaStream_t st);
 
 #define V1G_CUDA(h, call)                                                              \
   do {                                                                                 \
