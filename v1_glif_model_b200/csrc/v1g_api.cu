@@ -130,7 +130,7 @@ extern "C" int v1g_destroy(V1GHandle* h) {
   cudaFree(h->tref);
   cudaFree(h->basis);
   cudaFree(h->seg_counts);
-  cudaFree(h->coords);
+  cudaFree(h->gather_rows);
   cudaFree(h->d_count);
   if (h->h_count) cudaFreeHost(h->h_count);
   cudaFree(h->lgn_entries);

@@ -83,8 +83,8 @@ struct V1GHandle {
   // ---- scratch (grown on demand, freed in v1g_destroy) ----
   int32_t* seg_counts = nullptr;  // compaction: per-segment counts / offsets
   int64_t seg_cap = 0;
-  int64_t* coords = nullptr;  // op-level active list (row, col)
-  int64_t coords_cap = 0;
+  float* gather_rows = nullptr;  // op-level dx gather: output gradients laid out by (neuron, type or channel)
+  int64_t gather_rows_cap = 0;
   int32_t* d_count = nullptr;  // device int for counts
   int32_t* h_count = nullptr;  // pinned host mirror
   uint32_t* lgn_entries = nullptr;

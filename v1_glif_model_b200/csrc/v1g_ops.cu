@@ -14,27 +14,59 @@ struct DenseConsts {
 };
 
 // ------------------------------------------------------------------------------------------
-// spike -> current scatter over a compacted active list (models.py:134-169, 833-857, 896-934)
+// spike -> current scatter and weight gradient over the active columns (models.py:134-169, 833-857,
+// 896-934 and 226-240)
 // ------------------------------------------------------------------------------------------
+// A warp looks at `group` neighbouring columns of one batch row, and for every positive entry walks the
+// column's synapses; the positions never have to be listed, since nothing depends on their order (the
+// three launches of an ordered compaction, per source and call, were a sixth of the time of a step of
+// 5,000 neurons: 192 -> 162 us).  Sources
+// with few columns and long rows (background) are spread by taking one column per warp and every
+// `parts`-th pass of 32 synapses of its row.
+struct ActiveSplit {
+  int group, parts;
+  int64_t groups_per_row, items;
+};
+
+template <typename F>
+__device__ __forceinline__ void for_active(const ActiveSplit sp, const float* __restrict__ x, int64_t n_cols, int D, int n_src,
+                                           const int32_t* __restrict__ rowptr, F&& walk) {
+  const int lane = threadIdx.x & 31;
+  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t item = gw; item < sp.items; item += nw) {
+    const int part = (int)(item % sp.parts);
+    const int64_t g = item / sp.parts, b = g / sp.groups_per_row, c0 = (g - b * sp.groups_per_row) * sp.group;
+    const int64_t col = c0 + lane;
+    float xv = 0.f;
+    if (lane < sp.group && col < n_cols) xv = x[b * n_cols + col];
+    unsigned act = __ballot_sync(0xffffffffu, xv > 0.f);
+    int j0 = 0, j1 = 0;
+    if (xv > 0.f) {
+      const int64_t row = (D > 1) ? (col % n_src) * D + col / n_src : col;
+      j0 = rowptr[row];
+      j1 = rowptr[row + 1];
+    }
+    while (act) {
+      const int src = __ffs(act) - 1;
+      act &= act - 1;
+      const float mult = __shfl_sync(0xffffffffu, xv, src);
+      const int first = __shfl_sync(0xffffffffu, j0, src), end = __shfl_sync(0xffffffffu, j1, src);
+      walk(b, mult, first + 32 * part + lane, end, 32 * sp.parts);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) scatter_fwd_kernel(
-    const int64_t* __restrict__ coords, const int32_t* __restrict__ count,
-    const int32_t* __restrict__ rowptr, const int32_t* __restrict__ post,
+    const ActiveSplit sp, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ post,
     const float* __restrict__ w, const uint8_t* __restrict__ sid, const float* __restrict__ basis,
     const float* __restrict__ x, int64_t n_cols, int N, int R, int S, int D, int n_src, int is_bkg,
     float* __restrict__ i_flat) {
   extern __shared__ float basis_s[];
   for (int i = threadIdx.x; i < S * R; i += blockDim.x) basis_s[i] = basis[i];
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t n_act = *count;
-  for (int64_t e = gw; e < n_act; e += nw) {
-    const int64_t b = coords[2 * e], col = coords[2 * e + 1];
-    const int64_t row = (D > 1) ? (col % n_src) * D + col / n_src : col;
-    const float mult = is_bkg ? x[b * n_cols + col] : 1.f;
-    const int j1 = rowptr[row + 1];
-    for (int j = rowptr[row] + lane; j < j1; j += 32) {
+  for_active(sp, x, n_cols, D, n_src, rowptr, [&](int64_t b, float mult, int first, int end, int step) {
+    for (int j = first; j < end; j += step) {
       float wv = w[j];
       if (is_bkg) wv = wv * mult;  // (w * n_pre_spikes) * basis, models.py:931
       const float* bs = basis_s + (int)sid[j] * R;
@@ -44,62 +76,21 @@ __global__ void __launch_bounds__(256) scatter_fwd_kernel(
         if (c != 0.f) atomicAdd(dst + r, c);
       }
     }
-  }
-}
-
-// d_x[b, col] = sum over the synapses of column col of w * sum_r basis[sid,r]*dy[b,post,r]
-// (models.py:187-202; every synapse, active or not).
-__global__ void __launch_bounds__(256) gather_dx_kernel(
-    const int32_t* __restrict__ rowptr, const int32_t* __restrict__ post,
-    const float* __restrict__ w, const uint8_t* __restrict__ sid, const float* __restrict__ basis,
-    const float* __restrict__ dy, int64_t n_cols, int B, int N, int R, int S, int D, int n_src,
-    float* __restrict__ d_x) {
-  extern __shared__ float basis_s[];
-  for (int i = threadIdx.x; i < S * R; i += blockDim.x) basis_s[i] = basis[i];
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t total = (int64_t)B * n_cols;
-  for (int64_t e = gw; e < total; e += nw) {
-    const int64_t b = e / n_cols, col = e - b * n_cols;
-    const int64_t row = (D > 1) ? (col % n_src) * D + col / n_src : col;
-    const int j1 = rowptr[row + 1];
-    float acc = 0.f;
-    for (int j = rowptr[row] + lane; j < j1; j += 32) {
-      const float* bs = basis_s + (int)sid[j] * R;
-      const float* g = dy + (b * N + post[j]) * R;
-      const float wv = w[j];
-      float s = 0.f;
-      for (int r = 0; r < R; ++r) s += g[r] * (wv * bs[r]);
-      acc += s;
-    }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) d_x[e] = acc;
-  }
+  });
 }
 
 // d_w[syn] += sum_r dy[b,post,r]*basis[sid,r] for the synapses of active columns
 // (models.py:226-240); the background source carries the Poisson count (autodiff of :931).
 __global__ void __launch_bounds__(256) scatter_dw_kernel(
-    const int64_t* __restrict__ coords, const int32_t* __restrict__ count,
-    const int32_t* __restrict__ rowptr, const int32_t* __restrict__ post,
+    const ActiveSplit sp, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ post,
     const uint8_t* __restrict__ sid, const int32_t* __restrict__ perm,
     const float* __restrict__ basis, const float* __restrict__ x, const float* __restrict__ dy,
     int64_t n_cols, int N, int R, int S, int D, int n_src, int is_bkg, float* __restrict__ d_w) {
   extern __shared__ float basis_s[];
   for (int i = threadIdx.x; i < S * R; i += blockDim.x) basis_s[i] = basis[i];
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t n_act = *count;
-  for (int64_t e = gw; e < n_act; e += nw) {
-    const int64_t b = coords[2 * e], col = coords[2 * e + 1];
-    const int64_t row = (D > 1) ? (col % n_src) * D + col / n_src : col;
-    const float mult = is_bkg ? x[b * n_cols + col] : 1.f;
-    const int j1 = rowptr[row + 1];
-    for (int j = rowptr[row] + lane; j < j1; j += 32) {
+  for_active(sp, x, n_cols, D, n_src, rowptr, [&](int64_t b, float mult, int first, int end, int step) {
+    for (int j = first; j < end; j += step) {
       const float* bs = basis_s + (int)sid[j] * R;
       const float* g = dy + (b * N + post[j]) * R;
       float s = 0.f;
@@ -107,6 +98,118 @@ __global__ void __launch_bounds__(256) scatter_dw_kernel(
       if (is_bkg) s = s * mult;
       atomicAdd(d_w + perm[j], s);
     }
+  });
+}
+
+// ------------------------------------------------------------------------------------------
+// d_x[b, col] = sum over the synapses of column col of w * sum_r basis[sid,r]*dy[b,post,r]
+// (models.py:187-202; every synapse, active or not)
+// ------------------------------------------------------------------------------------------
+// Every synapse is read once for up to BP batch rows together.  What bounds the gather is one L2 sector
+// per synapse: dy is laid out anew so that the values one synapse needs are neighbours, padded to BP in
+// {1, 2, 4, 8} floats (32 bytes at most).  With few synapse types (PROJ) the basis is applied there too
+// and a synapse reads one such row, its type's; otherwise it reads the R rows of its target.  Currents and
+// both gradients of one step at 66,634 neurons, batch 5 (8 M synapses): 536 us with a pass over the
+// synapses per batch row, 157 us with this.
+constexpr int PROJ_MAX_TYPES = 8;
+
+template <int BP, bool PROJ>
+__global__ void __launch_bounds__(256) gather_rows_kernel(const float* __restrict__ dy, const float* __restrict__ basis,
+                                                          int b0, int nb, int N, int R, int S, float* __restrict__ rows) {
+  const int M = PROJ ? S : R;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)N * M; i += (int64_t)gridDim.x * blockDim.x) {
+    const int n = (int)(i / M), m = (int)(i - (int64_t)n * M);
+    float v[BP];
+#pragma unroll
+    for (int b = 0; b < BP; ++b) {
+      v[b] = 0.f;
+      if (b >= nb) continue;
+      const float* g = dy + ((int64_t)(b0 + b) * N + n) * R;
+      if (PROJ) {
+        for (int r = 0; r < R; ++r) v[b] += g[r] * basis[m * R + r];
+      } else {
+        v[b] = g[m];
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < BP; ++b) rows[i * BP + b] = v[b];
+  }
+}
+
+template <int BP>
+struct alignas(BP * 4 > 16 ? 16 : BP * 4) GatherRow {
+  float v[BP];
+};
+
+// LPR lanes walk one row of the CSR, U synapses each at a time with all their loads in flight
+template <int BP, bool PROJ, int LPR>
+__global__ void __launch_bounds__(256) gather_dx_kernel(
+    const int32_t* __restrict__ rowptr, const int32_t* __restrict__ post, const float* __restrict__ w,
+    const uint8_t* __restrict__ sid, const float* __restrict__ basis, const float* __restrict__ rows, int64_t n_cols, int b0,
+    int nb, int R, int S, int D, int n_src, float* __restrict__ d_x) {
+  constexpr int U = 4;
+  extern __shared__ float basis_s[];
+  if (!PROJ) {
+    for (int i = threadIdx.x; i < S * R; i += blockDim.x) basis_s[i] = basis[i];
+    __syncthreads();
+  }
+  const GatherRow<BP>* rw = reinterpret_cast<const GatherRow<BP>*>(rows);
+  const int l = threadIdx.x & (LPR - 1);
+  const int64_t g0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
+  const int64_t ng = ((int64_t)gridDim.x * blockDim.x) / LPR;
+  // whole warps stay in the loop, so that the shuffles below always have all their lanes
+  const int64_t n_it = (n_cols + ng - 1) / ng;
+  int64_t row = g0;
+  for (int64_t it = 0; it < n_it; ++it, row += ng) {
+    const bool in = row < n_cols;
+    const int j0 = in ? rowptr[row] : 0, j1 = in ? rowptr[row + 1] : 0;
+    float acc[BP];
+#pragma unroll
+    for (int b = 0; b < BP; ++b) acc[b] = 0.f;
+    for (int jb = j0 + l; jb < j1; jb += LPR * U) {
+      int p[U], s[U];
+      float wv[U];
+#pragma unroll
+      for (int q = 0; q < U; ++q) {
+        const int j = jb + q * LPR;
+        const bool ok = j < j1;
+        p[q] = ok ? post[j] : 0;
+        s[q] = ok ? (int)sid[j] : -1;
+        wv[q] = ok ? w[j] : 0.f;
+      }
+      if (PROJ) {
+        GatherRow<BP> gr[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+          if (s[q] >= 0) gr[q] = rw[(int64_t)p[q] * S + s[q]];
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+          if (s[q] >= 0) {
+#pragma unroll
+            for (int b = 0; b < BP; ++b) acc[b] += wv[q] * gr[q].v[b];
+          }
+      } else {
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          if (s[q] < 0) continue;
+          for (int r = 0; r < R; ++r) {
+            const float wb = wv[q] * basis_s[s[q] * R + r];
+            const GatherRow<BP> gr = rw[(int64_t)p[q] * R + r];
+#pragma unroll
+            for (int b = 0; b < BP; ++b) acc[b] += gr.v[b] * wb;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int b = 0; b < BP; ++b) acc[b] += __shfl_xor_sync(0xffffffffu, acc[b], o);
+    if (!in) continue;
+    const int64_t col = (D > 1) ? (row % D) * n_src + row / D : row;
+#pragma unroll
+    for (int b = 0; b < BP; ++b)
+      if (l == b && b < nb) d_x[(int64_t)(b0 + b) * n_cols + col] = acc[b];
   }
 }
 
@@ -225,17 +328,42 @@ int check_source(V1GHandle* h, int source, int batch) {
   return V1G_OK;
 }
 
-// compaction of x[B, n_cols] > 0 into h->coords / h->d_count
-int compact_active(V1GHandle* h, const float* x, int batch, int64_t n_cols, cudaStream_t st) {
-  const int nseg = (int)((n_cols + V1G_SEG - 1) / V1G_SEG);
+ActiveSplit split_active(const V1GHandle* h, const V1GSource& s, int batch) {
+  // about 32 warps per SM, each on as many columns as that leaves it (32 at most), and passes of 256
+  // synapses where a row is longer than that
+  const int64_t cols = (int64_t)batch * s.n_cols, warps = (int64_t)h->n_sms * 32;
+  ActiveSplit sp;
+  sp.group = 1;
+  while (sp.group < 32 && cols / sp.group > warps) sp.group *= 2;
+  const int64_t mean = s.n_cols > 0 ? s.nnz / s.n_cols : 0;
+  sp.parts = (int)std::min<int64_t>(std::max<int64_t>(mean / 256, 1), 64);
+  sp.groups_per_row = (s.n_cols + sp.group - 1) / sp.group;
+  sp.items = sp.groups_per_row * batch * sp.parts;
+  return sp;
+}
+
+unsigned active_blocks(const V1GHandle* h, const ActiveSplit& sp) {
+  return (unsigned)std::max<int64_t>(std::min<int64_t>((sp.items + 7) / 8, (int64_t)h->n_sms * 8), 1);
+}
+
+template <int BP, bool PROJ>
+int gather_dx(V1GHandle* h, const V1GSource& s, const float* dy, int b0, int nb, float* d_x, cudaStream_t st) {
+  const int N = h->cfg.n_neurons, R = h->cfg.n_receptors, S = h->cfg.n_syn_types;
+  const int64_t elems = (int64_t)N * (PROJ ? S : R);
   int rc;
-  if ((rc = v1g_reserve(h, &h->seg_counts, &h->seg_cap, (int64_t)batch * nseg + 1))) return rc;
-  if ((rc = v1g_reserve(h, &h->coords, &h->coords_cap, 2 * (int64_t)batch * n_cols))) return rc;
-  if ((rc = v1g_compact_count_scan(h, V1G_COMPACT_F32_COORDS, x, batch, n_cols, 0, h->seg_counts,
-                                   nullptr, st)))
-    return rc;
-  return v1g_compact_fill(h, V1G_COMPACT_F32_COORDS, x, batch, n_cols, 0, h->seg_counts, h->coords,
-                          (int64_t)batch * n_cols, st);
+  if ((rc = v1g_reserve(h, &h->gather_rows, &h->gather_rows_cap, elems * BP))) return rc;
+  gather_rows_kernel<BP, PROJ><<<(unsigned)std::min<int64_t>((elems + 255) / 256, (int64_t)h->n_sms * 8), 256, 0, st>>>(
+      dy, h->basis, b0, nb, N, R, S, h->gather_rows);
+  const size_t smem = PROJ ? 0 : (size_t)S * R * sizeof(float);
+  // rows of the recurrent source are short (one delay of one neuron): 8 lanes walk one, four rows per warp
+  const int lpr = s.nnz / std::max<int64_t>(s.n_cols, 1) < 48 ? 8 : 32;
+  const unsigned blocks = (unsigned)std::min<int64_t>((s.n_cols * lpr + 255) / 256, (int64_t)h->n_sms * 32);
+  auto kern = lpr == 8 ? gather_dx_kernel<BP, PROJ, 8> : gather_dx_kernel<BP, PROJ, 32>;
+  kern<<<blocks, 256, smem, st>>>(s.rowptr, s.post, s.w, s.sid, h->basis, h->gather_rows, s.n_cols, b0, nb, R, S, s.delays,
+                                  s.n_src, d_x);
+  v1g_count_launches(2);
+  V1G_CUDA(h, cudaGetLastError());
+  return V1G_OK;
 }
 
 }  // namespace
@@ -251,10 +379,10 @@ extern "C" int v1g_syn_currents_fwd(V1GHandle* h, int source, const float* x, in
   const int N = h->cfg.n_neurons, R = h->cfg.n_receptors, S = h->cfg.n_syn_types;
   V1G_CUDA(h, cudaMemsetAsync(i_flat, 0, (size_t)batch * N * R * sizeof(float), st));
   if (s.nnz == 0) return V1G_OK;
-  if ((rc = compact_active(h, x, batch, s.n_cols, st))) return rc;
-  scatter_fwd_kernel<<<h->n_sms * 4, 256, S * R * sizeof(float), st>>>(
-      h->coords, h->d_count, s.rowptr, s.post, s.w, s.sid, h->basis, x, s.n_cols, N, R, S, s.delays,
-      s.n_src, source == V1G_SRC_BKG, i_flat);
+  const ActiveSplit sp = split_active(h, s, batch);
+  scatter_fwd_kernel<<<active_blocks(h, sp), 256, S * R * sizeof(float), st>>>(
+      sp, s.rowptr, s.post, s.w, s.sid, h->basis, x, s.n_cols, N, R, S, s.delays, s.n_src,
+      source == V1G_SRC_BKG, i_flat);
   v1g_count_launches(1);
   V1G_CUDA(h, cudaGetLastError());
   return V1G_OK;
@@ -269,17 +397,24 @@ extern "C" int v1g_syn_currents_bwd(V1GHandle* h, int source, const float* x, co
   cudaStream_t st = (cudaStream_t)stream;
   const V1GSource& s = h->src[source];
   const int N = h->cfg.n_neurons, R = h->cfg.n_receptors, S = h->cfg.n_syn_types;
-  if (d_x) {
-    gather_dx_kernel<<<h->n_sms * 8, 256, S * R * sizeof(float), st>>>(
-        s.rowptr, s.post, s.w, s.sid, h->basis, dy, s.n_cols, batch, N, R, S, s.delays, s.n_src, d_x);
-    V1G_CUDA(h, cudaGetLastError());
+  if (d_x && s.n_cols > 0) {
+    const bool proj = S <= PROJ_MAX_TYPES;
+    for (int b0 = 0; b0 < batch; b0 += 8) {
+      const int nb = std::min(batch - b0, 8);
+      if (nb == 1) rc = proj ? gather_dx<1, true>(h, s, dy, b0, nb, d_x, st) : gather_dx<1, false>(h, s, dy, b0, nb, d_x, st);
+      else if (nb == 2) rc = proj ? gather_dx<2, true>(h, s, dy, b0, nb, d_x, st) : gather_dx<2, false>(h, s, dy, b0, nb, d_x, st);
+      else if (nb <= 4) rc = proj ? gather_dx<4, true>(h, s, dy, b0, nb, d_x, st) : gather_dx<4, false>(h, s, dy, b0, nb, d_x, st);
+      else rc = proj ? gather_dx<8, true>(h, s, dy, b0, nb, d_x, st) : gather_dx<8, false>(h, s, dy, b0, nb, d_x, st);
+      if (rc) return rc;
+    }
   }
   if (d_w && s.nnz > 0) {
     V1G_CUDA(h, cudaMemsetAsync(d_w, 0, (size_t)s.nnz * sizeof(float), st));
-    if ((rc = compact_active(h, x, batch, s.n_cols, st))) return rc;
-    scatter_dw_kernel<<<h->n_sms * 4, 256, S * R * sizeof(float), st>>>(
-        h->coords, h->d_count, s.rowptr, s.post, s.sid, s.perm, h->basis, x, dy, s.n_cols, N, R, S,
-        s.delays, s.n_src, source == V1G_SRC_BKG, d_w);
+    const ActiveSplit sp = split_active(h, s, batch);
+    scatter_dw_kernel<<<active_blocks(h, sp), 256, S * R * sizeof(float), st>>>(
+        sp, s.rowptr, s.post, s.sid, s.perm, h->basis, x, dy, s.n_cols, N, R, S, s.delays, s.n_src,
+        source == V1G_SRC_BKG, d_w);
+    v1g_count_launches(1);
     V1G_CUDA(h, cudaGetLastError());
   }
   return V1G_OK;
