@@ -133,3 +133,24 @@ def test_movie_to_column_activity_through_the_rates():
     cell.synchronize()
     assert int(x.sum()) > 0 and int(z1.sum()) > 0
     assert torch.equal(z1, z2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("height,width,sides,n_units,n_frames", [
+    (40, 70, tuple(range(1, 33, 2)), 300, 33),      # every patch width of the tiled kernel, two frame groups
+    (120, 240, (31,), 65, 1),                       # the widest tiled patch, one frame
+    (3, 5, (1, 3, 9), 40, 31),                      # patches larger than the frame
+    (40, 70, (5, 33), 300, 34),                     # one patch too wide for tiles: the per-stencil kernel
+    (24, 40, (3, 5), 4800, 521),                    # 32 outputs per thread in the temporal filter, ragged end
+])
+def test_device_matches_oracle_at_the_edges_of_the_tiled_kernel(height, width, sides, n_units, n_frames):
+    rng = np.random.Generator(np.random.PCG64(n_units + n_frames))
+    tb = random_tables(rng, n_units, height, width, sides, 40, 33)
+    movie = np.clip(rng.normal(0, 0.5, (n_frames, height, width)), -1, 1).astype(np.float32)
+    dom, non_dom = oracle_lgn.spatial_response(torch.from_numpy(movie).double(), tb)
+    want = oracle_lgn.firing_rates_from_spatial(dom, non_dom, tb)
+    lgn = device_lgn(tb, height, width)
+    got_dom, got_non_dom = lgn.spatial_response(movie)
+    close(got_dom.cpu(), dom)
+    close(got_non_dom.cpu(), non_dom)
+    close(lgn.firing_rates(movie).cpu(), want)

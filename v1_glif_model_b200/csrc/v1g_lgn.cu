@@ -12,19 +12,16 @@
 // tables are set: the four bilinear corners of the filtered frame are the same movie patch seen
 // through four shifted copies of the filter, each divided by its own edge normaliser, so
 //     response[t, u] = sum over a (k+1) x (k+1) patch of E[u][dy][dx] * movie[t, y0+dy, x0+dx]
-// with taps outside the frame dropped (they are the zero padding; their weights are stored as 0 and
-// the coordinates clamped, so the inner loop has no branch).  Stencils are sorted by side and stored
-// in groups of 32, one per lane of a warp, tap-major (weight of tap p of lane l at [p][l]), so a warp
-// reads one 128-byte line per tap and its lanes run the same trip count; inside a side they are
-// ordered so that the lanes of a group fall on different shared-memory banks.  A thread block takes two
-// frames, interleaved pixel by pixel, into shared memory (two 120 x 240 frames are 225 KB) and
-// evaluates every stencil on both from there: the movie is read from HBM once, a weight fetched from
-// L2 serves two frames, and one 8-byte shared-memory load brings both pixels.  The temporal filter
-// keeps a sliding window per thread: TT outputs of one unit per thread reuse every loaded sample and
-// kernel value TT times.
+// with taps outside the frame dropped (they are the zero padding; their weights are stored as 0).
+// Patches of up to 32 x 32 taps are evaluated by lgn_tile_kernel, a lane per frame; wider ones by
+// lgn_spatial_kernel, a lane per stencil.  The temporal filter keeps a sliding window per thread: TT
+// outputs of one unit per thread reuse every loaded sample and kernel value TT times.
 #include <math.h>
 
 #include <algorithm>
+#include <array>
+#include <map>
+#include <utility>
 #include <vector>
 
 #include "v1g_internal.h"
@@ -34,6 +31,13 @@ struct V1GLgn {
   int device = 0, n_sms = 0, smem_optin = 0;
   // stencils of the dominant [0, U) and non-dominant [U, 2U) subfields, sorted by side, 32 per group
   int n_groups = 0;
+  // patches of up to LGN_MAX_SIDE taps a side: tiles of the frame, see lgn_tile_kernel
+  int n_tiles = 0, tile_w = 0, tile_h = 0;
+  int2* tl_org = nullptr;      // [n_tiles] = (y, x) of the tile's first pixel
+  int4* tl_warp = nullptr;     // [n_tiles * 32] = (first stencil, end, first float4 of its weights, 0) per warp
+  int4* tl_st = nullptr;       // [2U] = (first pixel in the tile, side, subfield * U + unit, 0)
+  float4* tl_w = nullptr;      // weights, rows padded to whole float4, in the order of tl_st
+  // wider patches: groups of 32 stencils, see lgn_spatial_kernel
   int2* st_grp = nullptr;      // [n_groups] = (first tap of the group in st_w / 32, side)
   int4* st_slot = nullptr;     // [n_groups * 32] = (y0, x0, subfield * U + unit or -1 for an empty lane, 0)
   float* st_w = nullptr;       // per group [side * side][32]
@@ -65,7 +69,124 @@ int lgn_upload(V1GLgn* l, T** dst, const T* src, size_t n) {
   return V1G_OK;
 }
 
-// one block per F consecutive frames: they go to shared memory interleaved ([pixel][F]) and every
+__device__ __forceinline__ void cp_async_4_zfill(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(valid ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// Spatial responses, a lane per frame.  A block takes one tile of the frame for 32 frames into shared
+// memory as [pixel][frame] (33 words per pixel, so that both the transposing copy and the reads are free
+// of bank conflicts) and evaluates every stencil whose patch starts in the tile's cell: a warp walks one
+// patch, the 32 lanes read the 32 frames of a pixel in one wavefront, the weights are the same for all
+// lanes and the taps of a row have constant offsets.  Cells are as large as the shared memory allows for
+// the widest patch of the table (12 x 10 pixels for 30 x 30 taps); the tile overlaps its neighbours
+// by the patch width.
+// Bound by the shared-memory pipe: one wavefront per tap and 32 frames, and a quarter for the weights.
+// Weights stream from L2 (the whole table fits there) through a ring of 4 x 128 bytes per warp, three
+// lines ahead of the walk; every warp's stencils are consecutive in the table, so the stream does not
+// stop between stencils, and the host deals the stencils of a tile out over the warps by work.
+constexpr int LGN_MAX_SIDE = 32;
+constexpr int LGN_WARPS = 32;
+constexpr int LGN_PIX = 33;             // words per pixel
+constexpr int LGN_RING = 4 * 8;         // float4 per warp
+constexpr size_t LGN_RING_BYTES = (size_t)LGN_WARPS * LGN_RING * sizeof(float4);
+
+struct LgnStream {
+  const float4* src;   // next line of this warp's weights
+  float4* ring;
+  int issued;          // lines requested so far
+  int q;               // float4 consumed so far
+  // before a row of at most 8 float4: the lines q/8 and q/8 + 1 are in the ring, two more on their way
+  __device__ __forceinline__ void advance(int lane) {
+    const int c = q >> 3;
+    if (issued >= c + 4) return;
+    __syncwarp();      // every lane is through with the lines before c
+    do {
+      if (lane < 8) cp_async_16(ring + (issued & 3) * 8 + lane, src + issued * 8 + lane);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      ++issued;
+    } while (issued < c + 4);
+    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    __syncwarp();
+  }
+};
+
+template <int SIDE>
+__device__ __forceinline__ float lgn_walk(const float* px, int row_stride, LgnStream& ws, int lane) {
+  constexpr int NQ = (SIDE + 3) / 4;
+  float acc = 0.f;
+#pragma unroll 1
+  for (int dy = 0; dy < SIDE; ++dy) {
+    ws.advance(lane);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      const float4 w = ws.ring[(ws.q + i) & (LGN_RING - 1)];
+      acc += w.x * px[(4 * i) * LGN_PIX];
+      acc += w.y * px[(4 * i + 1) * LGN_PIX];
+      if (4 * i + 2 < SIDE) {
+        acc += w.z * px[(4 * i + 2) * LGN_PIX];
+        acc += w.w * px[(4 * i + 3) * LGN_PIX];
+      }
+    }
+    ws.q += NQ;
+    px += row_stride;
+  }
+  return acc;
+}
+
+__global__ void __launch_bounds__(32 * LGN_WARPS, 1)
+    lgn_tile_kernel(const float* __restrict__ movie, int T, int H, int W, int U, int n_tiles, int tile_h, int tile_w,
+                    const int2* __restrict__ tl_org, const int4* __restrict__ tl_warp, const int4* __restrict__ tl_st,
+                    const float4* __restrict__ tl_w, float* __restrict__ out) {
+  extern __shared__ __align__(128) float frame_s[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tile = (int)(blockIdx.x % (unsigned)n_tiles), t0 = (int)(blockIdx.x / (unsigned)n_tiles) * 32;
+  const int nf = min(32, T - t0);
+  float4* ring = reinterpret_cast<float4*>(frame_s) + warp * LGN_RING;
+  float* pix = frame_s + LGN_RING_BYTES / sizeof(float);
+  const int4 mine = tl_warp[tile * LGN_WARPS + warp];
+  const int2 org = tl_org[tile];
+  for (int i = warp; i < tile_h * nf; i += LGN_WARPS) {
+    const int f = i / tile_h, y = i - f * tile_h;
+    const int yy = org.x + y;
+    const bool row_in = yy >= 0 && yy < H;
+    const float* src = movie + ((int64_t)(t0 + f) * H + (row_in ? yy : 0)) * W;
+    for (int x = lane; x < tile_w; x += 32) {
+      const int xx = org.y + x;
+      const bool in = row_in && xx >= 0 && xx < W;
+      cp_async_4_zfill(pix + (y * tile_w + x) * LGN_PIX + f, src + (in ? xx : 0), in);   // outside the frame: 0
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  LgnStream ws{tl_w + mine.z, ring, 0, 0};
+  for (int k = mine.x; k < mine.y; ++k) {
+    const int4 st = tl_st[k];
+    const float* px = pix + (int64_t)st.x * LGN_PIX + lane;
+    const int rs = tile_w * LGN_PIX;
+    float acc = 0.f;
+    switch (st.y) {
+#define LGN_CASE(S) case S: acc = lgn_walk<S>(px, rs, ws, lane); break;
+      LGN_CASE(2) LGN_CASE(4) LGN_CASE(6) LGN_CASE(8) LGN_CASE(10) LGN_CASE(12) LGN_CASE(14) LGN_CASE(16)
+      LGN_CASE(18) LGN_CASE(20) LGN_CASE(22) LGN_CASE(24) LGN_CASE(26) LGN_CASE(28) LGN_CASE(30) LGN_CASE(32)
+#undef LGN_CASE
+    }
+    if (lane < nf) {
+      const int sub = st.z >= U ? 1 : 0, u = st.z - sub * U;
+      out[((int64_t)sub * T + t0 + lane) * U + u] = acc;
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Patches wider than LGN_MAX_SIDE.  Stencils are sorted by side and stored in groups of 32, one per lane
+// of a warp, tap-major (weight of tap p of lane l at [p][l]), so a warp reads one 128-byte line per tap
+// and its lanes run the same trip count; coordinates are clamped, so the inner loop has no branch.
+// One block per F consecutive frames: they go to shared memory interleaved ([pixel][F]) and every
 // stencil group is evaluated from there, one group per warp at a time; out[s][t][u].  With F == 1 and
 // IN_SMEM false (frames larger than shared memory) the pixels are read from global memory.
 constexpr int TB = 8;
@@ -131,10 +252,13 @@ __global__ void __launch_bounds__(1024) lgn_spatial_kernel(const float* __restri
 
 // rates[t][u] = relu(amp * f_dom + spont) + composite * relu(nd_amp * f_nd + spont), f = causal filter
 // of the unit's samples: f[t] = sum_j K[j] * s[t - (L - 1) + j] with s = 0 before the movie starts.
-// A thread owns TT consecutive outputs of one unit and walks the taps TT at a time over a window of
-// 2 TT samples held in registers: 2 TT loads feed TT * TT multiply-adds.
-constexpr int TT = 8;
-__global__ void __launch_bounds__(256) lgn_temporal_kernel(const float* __restrict__ spatial, int T, int U,
+// A thread owns TT consecutive outputs of one unit and walks the taps
+// TAPS at a time over a window of TT + TAPS samples held in registers: 2 TAPS loads feed TT * TAPS
+// multiply-adds.  What bounds it is the L2 traffic: the samples are read L / TT times and the
+// kernels T / TT times, 9 GB with 8 outputs per thread at 1000 frames of 17,400 units and 2.3 GB with 32.
+constexpr int TAPS = 8;
+template <int TT>
+__global__ void __launch_bounds__(128) lgn_temporal_kernel(const float* __restrict__ spatial, int T, int U,
                                                            const float* __restrict__ k_dom, int len_dom,
                                                            const float* __restrict__ k_nd, int len_nd,
                                                            const float* __restrict__ amp,
@@ -154,23 +278,24 @@ __global__ void __launch_bounds__(256) lgn_temporal_kernel(const float* __restri
 #pragma unroll
     for (int i = 0; i < TT; ++i) f[s][i] = 0.f;
     // output i, tap j reads sample t0 + i - (L - 1) + j; win[i + jj] is that sample for tap j0 + jj
-    float win[2 * TT];
+    float win[TT + TAPS];
     const int q0 = t0 - (L - 1);
 #pragma unroll
     for (int i = 0; i < TT; ++i) win[i] = sample(q0 + i);
-    for (int j0 = 0; j0 < L; j0 += TT) {
-      float kv[TT];
+#pragma unroll 1
+    for (int j0 = 0; j0 < L; j0 += TAPS) {
+      float kv[TAPS];
 #pragma unroll
-      for (int jj = 0; jj < TT; ++jj) {
+      for (int jj = 0; jj < TAPS; ++jj) {
         kv[jj] = j0 + jj < L ? kern[(int64_t)(j0 + jj) * U] : 0.f;
         win[TT + jj] = sample(q0 + j0 + TT + jj);
       }
 #pragma unroll
-      for (int jj = 0; jj < TT; ++jj)
+      for (int jj = 0; jj < TAPS; ++jj)
 #pragma unroll
         for (int i = 0; i < TT; ++i) f[s][i] += kv[jj] * win[i + jj];
 #pragma unroll
-      for (int i = 0; i < TT; ++i) win[i] = win[TT + i];
+      for (int i = 0; i < TT; ++i) win[i] = win[TAPS + i];
     }
   }
   const float a = amp[u], an = nd_amp[u], c = composite[u], sp = spont[u];
@@ -246,79 +371,147 @@ extern "C" int v1g_lgn_create(const V1GLgnTables* tb, V1GLgn** out) {
         st.w[(size_t)dy * side + dx] = inside ? (float)e[(size_t)dy * side + dx] : 0.f;
       }
   }
-  std::vector<int> order((size_t)2 * U);
-  for (int i = 0; i < 2 * U; ++i) order[i] = i;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sts[a].side < sts[b].side; });
-  // Bank conflicts.  The 32 lanes of a group read the same tap (dy, dx) of 32 different patches, so the
-  // shared-memory bank of a lane is fixed by its patch corner: (y0 * W + x0) modulo M, M = 16 pixel
-  // pairs when two frames are interleaved (a half warp per wavefront), 32 pixels with one frame.
-  // Within a run of equal side the stencils are therefore dealt out round-robin over the M residues,
-  // so that (almost) every M consecutive lanes hit M different banks: an 8-byte load then takes
-  // about 2 wavefronts instead of the 6 that randomly placed patches take (5.7 -> 4.1 ms per 1000
-  // frames of 17,400 units).  Measured on top of it and slower: a branch for groups whose patches
-  // all lie inside the frame (no clamping, tap offsets from a table per side; 4.8 ms, the groups
-  // that cross the edge then cluster), and a warp per stencil with its lanes on consecutive taps
-  // (12.5 ms: one stencil's dependent loads at a time per warp).
-  {
-    cudaDeviceProp prop0;
-    int dev0 = 0;
-    if (cudaGetDevice(&dev0) != cudaSuccess || cudaGetDeviceProperties(&prop0, dev0) != cudaSuccess)
-      return lgn_fail(nullptr, V1G_ECUDA, "v1g_lgn_create: no CUDA device");
-    const int M = 2 * (size_t)H * W * sizeof(float) <= prop0.sharedMemPerBlockOptin ? 16 : 32;
-    std::vector<int> dealt;
-    dealt.reserve(order.size());
-    for (size_t lo = 0; lo < order.size();) {
-      size_t hi = lo;
-      while (hi < order.size() && sts[order[hi]].side == sts[order[lo]].side) ++hi;
-      std::vector<std::vector<int>> bucket((size_t)M);
-      for (size_t i = lo; i < hi; ++i) {
-        const Stencil& st = sts[order[i]];
-        const long long key = (long long)st.y0 * W + st.x0;
-        bucket[(size_t)(((key % M) + M) % M)].push_back(order[i]);
-      }
-      for (size_t round = 0, left = hi - lo; left > 0; ++round)
-        for (int r = 0; r < M; ++r)
-          if (round < bucket[(size_t)r].size()) {
-            dealt.push_back(bucket[(size_t)r][round]);
-            --left;
-          }
-      lo = hi;
+  cudaDeviceProp prop;
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || cudaGetDeviceProperties(&prop, device) != cudaSuccess)
+    return lgn_fail(nullptr, V1G_ECUDA, "v1g_lgn_create: no CUDA device");
+  int max_side = 0, x_min = INT32_MAX, y_min = INT32_MAX;
+  for (const Stencil& st : sts) {
+    max_side = std::max(max_side, st.side);
+    x_min = std::min(x_min, st.x0);
+    y_min = std::min(y_min, st.y0);
+  }
+  // ---- tiles: patches of at most LGN_MAX_SIDE taps a side ----
+  // The line lies there because a row of a patch is read from a ring of four lines per warp and may span
+  // two of them, and because the cell shrinks to nothing as the patch approaches the tile.
+  std::vector<int2> tl_org;
+  std::vector<int4> tl_warp, tl_st;
+  std::vector<float> tl_w;
+  int tile_w = 0, tile_h = 0;
+  const bool tiled = max_side <= LGN_MAX_SIDE;
+  if (tiled) {
+    const int cap = (int)((prop.sharedMemPerBlockOptin - LGN_RING_BYTES) / (LGN_PIX * sizeof(float)));
+    int cw = 0, ch = 0;      // cell: the patch corners a tile serves
+    for (int w = 1; w <= W + max_side; ++w) {
+      const int h = std::min(cap / (w + max_side - 1) - max_side + 1, H + max_side);
+      if (h >= 1 && w * h > cw * ch) { cw = w; ch = h; }
     }
-    order.swap(dealt);
+    if (cw == 0) return lgn_fail(nullptr, V1G_ERANGE, "v1g_lgn_create: no room for a tile in shared memory");
+    tile_w = cw + max_side - 1;
+    tile_h = ch + max_side - 1;
+    std::map<std::pair<int, int>, std::vector<int>> cells;
+    for (int i = 0; i < 2 * U; ++i) cells[{(sts[i].y0 - y_min) / ch, (sts[i].x0 - x_min) / cw}].push_back(i);
+    int64_t n4 = 0;
+    for (auto& cell : cells) {
+      const int ty = y_min + cell.first.first * ch, tx = x_min + cell.first.second * cw;
+      tl_org.push_back(make_int2(ty, tx));
+      // longest first, each to the warp with the least work (taps + what a row and a stencil cost besides)
+      std::vector<int>& ids = cell.second;
+      std::stable_sort(ids.begin(), ids.end(), [&](int a, int b) { return sts[a].side > sts[b].side; });
+      std::vector<int> list[LGN_WARPS];
+      std::array<int64_t, LGN_WARPS> load{};
+      for (int i : ids) {
+        const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        list[w].push_back(i);
+        load[w] += (int64_t)sts[i].side * (sts[i].side + 4) + 20;
+      }
+      for (int w = 0; w < LGN_WARPS; ++w) {
+        const int first = (int)tl_st.size();
+        const int64_t first4 = n4;
+        for (int i : list[w]) {
+          const Stencil& st = sts[i];
+          const int nq = (st.side + 3) / 4;
+          tl_st.push_back(make_int4((st.y0 - ty) * tile_w + st.x0 - tx, st.side, i, 0));
+          tl_w.resize((size_t)(n4 + (int64_t)nq * st.side) * 4, 0.f);
+          for (int dy = 0; dy < st.side; ++dy)
+            for (int dx = 0; dx < st.side; ++dx)
+              tl_w[(size_t)(n4 + (int64_t)dy * nq) * 4 + dx] = st.w[(size_t)dy * st.side + dx];
+          n4 += (int64_t)nq * st.side;
+        }
+        if (n4 > INT32_MAX / 2) return lgn_fail(nullptr, V1G_EINVAL, "v1g_lgn_create: stencil table too large");
+        tl_warp.push_back(make_int4(first, (int)tl_st.size(), (int)first4, 0));
+      }
+    }
+    tl_w.resize(tl_w.size() + 4 * 8 * 5, 0.f);   // the last warp's stream is requested up to four lines past its end
   }
-  const int n_groups = (2 * U + 31) / 32;
-  std::vector<int2> grp((size_t)n_groups);
-  std::vector<int4> slot((size_t)n_groups * 32, make_int4(0, 0, -1, 0));
-  int64_t taps = 0;
-  for (int gi = 0; gi < n_groups; ++gi) {
-    const int last = std::min(2 * U, (gi + 1) * 32) - 1;
-    grp[gi] = make_int2((int)taps, sts[order[last]].side);   // sorted: the last lane has the widest patch
-    taps += ((int64_t)grp[gi].y * grp[gi].y + TB - 1) / TB * TB;   // padded with zero weights
-  }
-  if (taps * 32 > (int64_t)INT32_MAX) return lgn_fail(nullptr, V1G_EINVAL, "v1g_lgn_create: stencil table too large");
-  std::vector<float> w((size_t)taps * 32, 0.f);
-  for (int i = 0; i < 2 * U; ++i) {
-    const int gi = i >> 5, ln = i & 31, gside = grp[gi].y;
-    const Stencil& st = sts[order[i]];
-    slot[i] = make_int4(st.y0, st.x0, order[i], 0);
-    // a narrower stencil sits in the top-left corner of the group's patch; the rest stays 0
-    for (int dy = 0; dy < st.side; ++dy)
-      for (int dx = 0; dx < st.side; ++dx)
-        w[((size_t)grp[gi].x + (size_t)dy * gside + dx) * 32 + ln] = st.w[(size_t)dy * st.side + dx];
+  // ---- groups of 32 stencils: wider patches ----
+  std::vector<int2> grp;
+  std::vector<int4> slot;
+  std::vector<float> w;
+  int n_groups = 0;
+  if (!tiled) {
+    std::vector<int> order((size_t)2 * U);
+    for (int i = 0; i < 2 * U; ++i) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sts[a].side < sts[b].side; });
+    // Bank conflicts.  The 32 lanes of a group read the same tap (dy, dx) of 32 different patches, so the
+    // shared-memory bank of a lane is fixed by its patch corner: (y0 * W + x0) modulo M, M = 16 pixel
+    // pairs when two frames are interleaved (a half warp per wavefront), 32 pixels with one frame.
+    // Within a run of equal side the stencils are therefore dealt out round-robin over the M residues,
+    // so that (almost) every M consecutive lanes hit M different banks: an 8-byte load then takes
+    // about 2 wavefronts instead of the 6 that randomly placed patches take (5.7 -> 4.1 ms per 1000
+    // frames of 17,400 units).  Measured on top of it and slower: a branch for groups whose patches
+    // all lie inside the frame (no clamping, tap offsets from a table per side; 4.8 ms, the groups
+    // that cross the edge then cluster), and a warp per stencil with its lanes on consecutive taps
+    // (12.5 ms: one stencil's dependent loads at a time per warp).
+    {
+      const int M = 2 * (size_t)H * W * sizeof(float) <= prop.sharedMemPerBlockOptin ? 16 : 32;
+      std::vector<int> dealt;
+      dealt.reserve(order.size());
+      for (size_t lo = 0; lo < order.size();) {
+        size_t hi = lo;
+        while (hi < order.size() && sts[order[hi]].side == sts[order[lo]].side) ++hi;
+        std::vector<std::vector<int>> bucket((size_t)M);
+        for (size_t i = lo; i < hi; ++i) {
+          const Stencil& st = sts[order[i]];
+          const long long key = (long long)st.y0 * W + st.x0;
+          bucket[(size_t)(((key % M) + M) % M)].push_back(order[i]);
+        }
+        for (size_t round = 0, left = hi - lo; left > 0; ++round)
+          for (int r = 0; r < M; ++r)
+            if (round < bucket[(size_t)r].size()) {
+              dealt.push_back(bucket[(size_t)r][round]);
+              --left;
+            }
+        lo = hi;
+      }
+      order.swap(dealt);
+    }
+    n_groups = (2 * U + 31) / 32;
+    grp.resize((size_t)n_groups);
+    slot.assign((size_t)n_groups * 32, make_int4(0, 0, -1, 0));
+    int64_t taps = 0;
+    for (int gi = 0; gi < n_groups; ++gi) {
+      const int last = std::min(2 * U, (gi + 1) * 32) - 1;
+      grp[gi] = make_int2((int)taps, sts[order[last]].side);   // sorted: the last lane has the widest patch
+      taps += ((int64_t)grp[gi].y * grp[gi].y + TB - 1) / TB * TB;   // padded with zero weights
+    }
+    if (taps * 32 > (int64_t)INT32_MAX) return lgn_fail(nullptr, V1G_EINVAL, "v1g_lgn_create: stencil table too large");
+    w.assign((size_t)taps * 32, 0.f);
+    for (int i = 0; i < 2 * U; ++i) {
+      const int gi = i >> 5, ln = i & 31, gside = grp[gi].y;
+      const Stencil& st = sts[order[i]];
+      slot[i] = make_int4(st.y0, st.x0, order[i], 0);
+      // a narrower stencil sits in the top-left corner of the group's patch; the rest stays 0
+      for (int dy = 0; dy < st.side; ++dy)
+        for (int dx = 0; dx < st.side; ++dx)
+          w[((size_t)grp[gi].x + (size_t)dy * gside + dx) * 32 + ln] = st.w[(size_t)dy * st.side + dx];
+    }
   }
 
   V1GLgn* l = new V1GLgn();
   l->n_units = U; l->height = H; l->width = W; l->len_dom = tb->len_dom; l->len_non_dom = tb->len_non_dom;
-  cudaDeviceProp prop;
-  if (cudaGetDevice(&l->device) != cudaSuccess || cudaGetDeviceProperties(&prop, l->device) != cudaSuccess) {
-    delete l;
-    return lgn_fail(nullptr, V1G_ECUDA, "v1g_lgn_create: no CUDA device");
-  }
+  l->device = device;
   l->n_sms = prop.multiProcessorCount;
   l->smem_optin = (int)prop.sharedMemPerBlockOptin;
   int rc = V1G_OK;
   l->n_groups = n_groups;
-  if ((rc = lgn_upload(l, &l->st_grp, grp.data(), grp.size())) || (rc = lgn_upload(l, &l->st_slot, slot.data(), slot.size())) ||
+  l->n_tiles = (int)tl_org.size();
+  l->tile_w = tile_w;
+  l->tile_h = tile_h;
+  if ((rc = lgn_upload(l, &l->tl_org, tl_org.data(), tl_org.size())) || (rc = lgn_upload(l, &l->tl_warp, tl_warp.data(), tl_warp.size())) ||
+      (rc = lgn_upload(l, &l->tl_st, tl_st.data(), tl_st.size())) ||
+      (rc = lgn_upload(l, &l->tl_w, reinterpret_cast<const float4*>(tl_w.data()), tl_w.size() / 4)) ||
+      (rc = lgn_upload(l, &l->st_grp, grp.data(), grp.size())) || (rc = lgn_upload(l, &l->st_slot, slot.data(), slot.size())) ||
       (rc = lgn_upload(l, &l->st_w, w.data(), w.size())) ||
       (rc = lgn_upload(l, &l->k_dom, tb->dom_temporal_kernels, (size_t)tb->len_dom * U)) ||
       (rc = lgn_upload(l, &l->k_non_dom, tb->non_dom_temporal_kernels, (size_t)tb->len_non_dom * U)) ||
@@ -335,6 +528,7 @@ extern "C" int v1g_lgn_create(const V1GLgnTables* tb, V1GLgn** out) {
 
 extern "C" int v1g_lgn_destroy(V1GLgn* l) {
   if (!l) return V1G_OK;
+  cudaFree(l->tl_org); cudaFree(l->tl_warp); cudaFree(l->tl_st); cudaFree(l->tl_w);
   cudaFree(l->st_grp); cudaFree(l->st_slot); cudaFree(l->st_w); cudaFree(l->k_dom); cudaFree(l->k_non_dom);
   cudaFree(l->amp); cudaFree(l->non_dom_amp); cudaFree(l->composite); cudaFree(l->spont); cudaFree(l->spatial);
   delete l;
@@ -362,7 +556,16 @@ extern "C" int v1g_lgn_firing_rates(V1GLgn* l, const float* movie, int32_t n_fra
     spatial = l->spatial;
   }
   const size_t frame_bytes = (size_t)l->height * l->width * sizeof(float);
-  if (movie) {
+  if (movie && l->n_tiles > 0) {
+    const size_t smem = LGN_RING_BYTES + (size_t)l->tile_w * l->tile_h * LGN_PIX * sizeof(float);
+    LGN_CUDA(l, cudaFuncSetAttribute(lgn_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t blocks = (int64_t)l->n_tiles * ((T + 31) / 32);
+    if (blocks > INT32_MAX) return lgn_fail(l, V1G_EINVAL, "v1g_lgn_firing_rates: movie too long");
+    lgn_tile_kernel<<<(unsigned)blocks, 32 * LGN_WARPS, smem, st>>>(movie, T, l->height, l->width, U, l->n_tiles, l->tile_h,
+                                                                    l->tile_w, l->tl_org, l->tl_warp, l->tl_st, l->tl_w,
+                                                                    spatial);
+    v1g_count_launches(1);
+  } else if (movie) {
     const int F = 2 * frame_bytes <= (size_t)l->smem_optin ? 2 : 1;
     const int in_smem = (size_t)F * frame_bytes <= (size_t)l->smem_optin ? 1 : 0;
     const size_t smem = in_smem ? F * frame_bytes : 0;
@@ -374,9 +577,12 @@ extern "C" int v1g_lgn_firing_rates(V1GLgn* l, const float* movie, int32_t n_fra
     v1g_count_launches(1);
   }
   if (rates_out) {
-    dim3 grid((U + 255) / 256, (T + TT - 1) / TT);
-    lgn_temporal_kernel<<<grid, 256, 0, st>>>(spatial, T, U, l->k_dom, l->len_dom, l->k_non_dom, l->len_non_dom, l->amp,
-                                              l->non_dom_amp, l->composite, l->spont, rates_out);
+    // 32 outputs per thread where that still gives every SM four blocks, else 8
+    const int ub = (U + 127) / 128, tt = (int64_t)ub * ((T + 31) / 32) >= 4 * (int64_t)l->n_sms ? 32 : 8;
+    const dim3 grid(ub, (T + tt - 1) / tt);
+    auto kern = tt == 32 ? lgn_temporal_kernel<32> : lgn_temporal_kernel<8>;
+    kern<<<grid, 128, 0, st>>>(spatial, T, U, l->k_dom, l->len_dom, l->k_non_dom, l->len_non_dom, l->amp, l->non_dom_amp,
+                               l->composite, l->spont, rates_out);
     v1g_count_launches(1);
   }
   LGN_CUDA(l, cudaGetLastError());
