@@ -681,7 +681,7 @@ static int rollout_fwd_impl(V1GHandle* h, int32_t batch, int32_t n_steps, const 
   // Register-resident kernel when the slice fits one neuron per thread and the (R, B) pair is
   // instantiated; the shared-memory kernel otherwise.
   const bool reg_ok = !h->opt_force_smem_kernel && !h->opt_force_global && plan.chunk <= V1G_NT_REG &&
-                      (R == 4 || R == 5) && B <= 6 &&
+                      (R == 4 || R == 5) &&
                       v1g_fwd_reg_smem(h, B, plan.chunkP, bkg_cap) <= limit;
   a.slice = nullptr;
   if (reg_ok && sliced && v1g_fwd_reg_smem(h, B, plan.chunkP, bkg_cap_sliced) <= limit) {
