@@ -85,32 +85,36 @@ __device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
 // the widest patch of the table (12 x 10 pixels for 30 x 30 taps); the tile overlaps its neighbours
 // by the patch width.
 // Bound by the shared-memory pipe: one wavefront per tap and 32 frames, and a quarter for the weights.
-// Weights stream from L2 (the whole table fits there) through a ring of 4 x 128 bytes per warp, three
-// lines ahead of the walk; every warp's stencils are consecutive in the table, so the stream does not
-// stop between stencils, and the host deals the stencils of a tile out over the warps by work.
+// Weights stream from L2 (the whole table fits there) through two units of 256 bytes per warp, one in use
+// and one on its way; every warp's stencils are consecutive in the table, so the stream does not stop
+// between stencils, and the host deals the stencils of a tile out over the warps by work.
 constexpr int LGN_MAX_SIDE = 32;
 constexpr int LGN_WARPS = 32;
 constexpr int LGN_PIX = 33;             // words per pixel
-constexpr int LGN_RING = 4 * 8;         // float4 per warp
+constexpr int LGN_UNIT = 16;            // float4 of weights requested together; a row lies in one unit
+constexpr int LGN_RING = 2 * LGN_UNIT;  // float4 per warp
 constexpr size_t LGN_RING_BYTES = (size_t)LGN_WARPS * LGN_RING * sizeof(float4);
 
 struct LgnStream {
-  const float4* src;   // next line of this warp's weights
+  const float4* next;   // unit to request
   float4* ring;
-  int issued;          // lines requested so far
-  int q;               // float4 consumed so far
-  // before a row of at most 8 float4: the lines q/8 and q/8 + 1 are in the ring, two more on their way
-  __device__ __forceinline__ void advance(int lane) {
-    const int c = q >> 3;
-    if (issued >= c + 4) return;
-    __syncwarp();      // every lane is through with the lines before c
-    do {
-      if (lane < 8) cp_async_16(ring + (issued & 3) * 8 + lane, src + issued * 8 + lane);
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      ++issued;
-    } while (issued < c + 4);
-    asm volatile("cp.async.wait_group 2;" ::: "memory");
+  const float4* at;     // weights of the next row
+  int left;             // float4 left in the current unit
+  unsigned half;        // half of the ring that holds the current unit
+  __device__ __forceinline__ void request(int lane, unsigned to) {
+    if (lane < LGN_UNIT) cp_async_16(ring + to * LGN_UNIT + lane, next + lane);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    next += LGN_UNIT;
+  }
+  // the current unit holds no further row: on to the other half, and refill this one
+  __device__ __forceinline__ void turn(int lane) {
+    __syncwarp();      // every lane is through with the current unit
+    request(lane, half);
+    half ^= 1u;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
+    at = ring + half * LGN_UNIT;
+    left = LGN_UNIT;
   }
 };
 
@@ -120,10 +124,10 @@ __device__ __forceinline__ float lgn_walk(const float* px, int row_stride, LgnSt
   float acc = 0.f;
 #pragma unroll 1
   for (int dy = 0; dy < SIDE; ++dy) {
-    ws.advance(lane);
+    if (ws.left < NQ) ws.turn(lane);
 #pragma unroll
     for (int i = 0; i < NQ; ++i) {
-      const float4 w = ws.ring[(ws.q + i) & (LGN_RING - 1)];
+      const float4 w = ws.at[i];
       acc += w.x * px[(4 * i) * LGN_PIX];
       acc += w.y * px[(4 * i + 1) * LGN_PIX];
       if (4 * i + 2 < SIDE) {
@@ -131,7 +135,8 @@ __device__ __forceinline__ float lgn_walk(const float* px, int row_stride, LgnSt
         acc += w.w * px[(4 * i + 3) * LGN_PIX];
       }
     }
-    ws.q += NQ;
+    ws.at += NQ;
+    ws.left -= NQ;
     px += row_stride;
   }
   return acc;
@@ -149,21 +154,23 @@ __global__ void __launch_bounds__(32 * LGN_WARPS, 1)
   float* pix = frame_s + LGN_RING_BYTES / sizeof(float);
   const int4 mine = tl_warp[tile * LGN_WARPS + warp];
   const int2 org = tl_org[tile];
-  for (int i = warp; i < tile_h * nf; i += LGN_WARPS) {
-    const int f = i / tile_h, y = i - f * tile_h;
-    const int yy = org.x + y;
-    const bool row_in = yy >= 0 && yy < H;
-    const float* src = movie + ((int64_t)(t0 + f) * H + (row_in ? yy : 0)) * W;
+  LgnStream ws{tl_w + mine.z, ring, nullptr, 0, 1u};
+  ws.request(lane, 0);
+  // a warp per frame; what lies outside the frame is 0
+  if (warp < nf) {
+    const float* src = movie + ((int64_t)(t0 + warp) * H + org.x) * W + org.y;
+    float* dst = pix + warp;
     for (int x = lane; x < tile_w; x += 32) {
-      const int xx = org.y + x;
-      const bool in = row_in && xx >= 0 && xx < W;
-      cp_async_4_zfill(pix + (y * tile_w + x) * LGN_PIX + f, src + (in ? xx : 0), in);   // outside the frame: 0
+      const bool col_in = org.y + x >= 0 && org.y + x < W;
+      for (int y = 0; y < tile_h; ++y) {
+        const bool in = col_in && org.x + y >= 0 && org.x + y < H;
+        cp_async_4_zfill(dst + (y * tile_w + x) * LGN_PIX, in ? src + (int64_t)y * W + x : movie, in);
+      }
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  LgnStream ws{tl_w + mine.z, ring, 0, 0};
   for (int k = mine.x; k < mine.y; ++k) {
     const int4 st = tl_st[k];
     const float* px = pix + (int64_t)st.x * LGN_PIX + lane;
@@ -282,14 +289,25 @@ __global__ void __launch_bounds__(128) lgn_temporal_kernel(const float* __restri
     const int q0 = t0 - (L - 1);
 #pragma unroll
     for (int i = 0; i < TT; ++i) win[i] = sample(q0 + i);
+    // kernel values and samples of a round are requested one round ahead
+    float kn[TAPS], sn[TAPS];
+    auto request = [&](int j0) {
+#pragma unroll
+      for (int jj = 0; jj < TAPS; ++jj) {
+        kn[jj] = j0 + jj < L ? kern[(int64_t)(j0 + jj) * U] : 0.f;
+        sn[jj] = sample(q0 + j0 + TT + jj);
+      }
+    };
+    request(0);
 #pragma unroll 1
     for (int j0 = 0; j0 < L; j0 += TAPS) {
       float kv[TAPS];
 #pragma unroll
       for (int jj = 0; jj < TAPS; ++jj) {
-        kv[jj] = j0 + jj < L ? kern[(int64_t)(j0 + jj) * U] : 0.f;
-        win[TT + jj] = sample(q0 + j0 + TT + jj);
+        kv[jj] = kn[jj];
+        win[TT + jj] = sn[jj];
       }
+      if (j0 + TAPS < L) request(j0 + TAPS);
 #pragma unroll
       for (int jj = 0; jj < TAPS; ++jj)
 #pragma unroll
@@ -382,8 +400,8 @@ extern "C" int v1g_lgn_create(const V1GLgnTables* tb, V1GLgn** out) {
     y_min = std::min(y_min, st.y0);
   }
   // ---- tiles: patches of at most LGN_MAX_SIDE taps a side ----
-  // The line lies there because a row of a patch is read from a ring of four lines per warp and may span
-  // two of them, and because the cell shrinks to nothing as the patch approaches the tile.
+  // The line lies there because the cell shrinks to nothing as the patch approaches the tile: 9 x 9 pixels
+  // for 32 x 32 taps, 4 x 4 for 37 x 37.
   std::vector<int2> tl_org;
   std::vector<int4> tl_warp, tl_st;
   std::vector<float> tl_w;
@@ -418,21 +436,28 @@ extern "C" int v1g_lgn_create(const V1GLgnTables* tb, V1GLgn** out) {
       for (int w = 0; w < LGN_WARPS; ++w) {
         const int first = (int)tl_st.size();
         const int64_t first4 = n4;
+        int left = LGN_UNIT;
         for (int i : list[w]) {
           const Stencil& st = sts[i];
           const int nq = (st.side + 3) / 4;
           tl_st.push_back(make_int4((st.y0 - ty) * tile_w + st.x0 - tx, st.side, i, 0));
-          tl_w.resize((size_t)(n4 + (int64_t)nq * st.side) * 4, 0.f);
-          for (int dy = 0; dy < st.side; ++dy)
-            for (int dx = 0; dx < st.side; ++dx)
-              tl_w[(size_t)(n4 + (int64_t)dy * nq) * 4 + dx] = st.w[(size_t)dy * st.side + dx];
-          n4 += (int64_t)nq * st.side;
+          for (int dy = 0; dy < st.side; ++dy) {
+            if (left < nq) {   // as LgnStream::turn: a row does not cross the end of a unit
+              n4 += left;
+              left = LGN_UNIT;
+            }
+            tl_w.resize((size_t)(n4 + nq) * 4, 0.f);
+            for (int dx = 0; dx < st.side; ++dx) tl_w[(size_t)n4 * 4 + dx] = st.w[(size_t)dy * st.side + dx];
+            n4 += nq;
+            left -= nq;
+          }
         }
+        n4 = (n4 + LGN_UNIT - 1) / LGN_UNIT * LGN_UNIT;
         if (n4 > INT32_MAX / 2) return lgn_fail(nullptr, V1G_EINVAL, "v1g_lgn_create: stencil table too large");
         tl_warp.push_back(make_int4(first, (int)tl_st.size(), (int)first4, 0));
       }
     }
-    tl_w.resize(tl_w.size() + 4 * 8 * 5, 0.f);   // the last warp's stream is requested up to four lines past its end
+    tl_w.resize((size_t)(n4 + 2 * LGN_UNIT) * 4, 0.f);   // a stream is requested one unit past its end
   }
   // ---- groups of 32 stencils: wider patches ----
   std::vector<int2> grp;
