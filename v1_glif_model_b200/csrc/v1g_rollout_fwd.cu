@@ -654,6 +654,7 @@ static int rollout_fwd_impl(V1GHandle* h, int32_t batch, int32_t n_steps, const 
     a.pinit[r] = r < R ? h->psc_initial[r] : 0.f;
     a.dtsd[r] = c.dt * a.sd[r];
   }
+  a.minus_zero2 = 0x8000000080000000ull;
   a.lr_scale = c.lr_scale; a.vd_keep = h->vd_keep; a.vd_drop = h->vd_drop;
   a.hard_reset = (c.flags & V1G_FLAG_HARD_RESET) ? 1 : 0;
   a.lgn_off = h->lgn_offsets; a.lgn_entries = h->lgn_entries; a.lgn_ent4 = h->lgn_ent4; a.lgn_nseg = nseg;

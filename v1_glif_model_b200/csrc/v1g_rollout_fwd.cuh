@@ -21,6 +21,7 @@ struct FwdArgs {
   const int32_t* tref;
   float sd[V1G_MAX_RECEPTORS], pinit[V1G_MAX_RECEPTORS], dtsd[V1G_MAX_RECEPTORS];
   float lr_scale, vd_keep, vd_drop;
+  unsigned long long minus_zero2;  // two floats of -0
   int hard_reset;
   // inputs
   const int32_t* lgn_off;  // exclusive offsets per (t, b, seg) segment

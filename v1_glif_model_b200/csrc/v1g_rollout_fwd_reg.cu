@@ -24,7 +24,7 @@ constexpr int NT = V1G_NT_REG;
 constexpr int NW = NT / 32;
 // State that a thread touches once per row and step lives in shared memory instead of registers (128 per
 // thread): psc_rise always; the after-spike currents up to 6 rows, psc from 7 rows on (both together
-// would not fit for 8 rows of 5 channels).  8 rows take 16.7 us per step at 66,634 neurons; the
+// would not fit for 8 rows of 5 channels).  8 rows take 16.5 us per step at 66,634 neurons; the
 // shared-memory kernel, which has no registers to spill but walks the rows one after another, took 30.2.
 __host__ __device__ constexpr bool asc_in_smem(int B) { return B <= 6; }
 __host__ __device__ constexpr bool psc_in_smem(int B) { return B > 6; }
@@ -33,8 +33,8 @@ __host__ __device__ constexpr bool psc_in_smem(int B) { return B > 6; }
 // (each rounded on its own, so the results are those of the scalar operations), and what the rows
 // share - background synapses, basis rows, constants - is read once.  A last odd row goes alone.  The
 // dense phase is bound by instruction issue, 15 warps per SM with one neuron per thread; microseconds per
-// step one row at a time and in pairs, 66,634 neurons at 4 Hz: batch 5 10.00 -> 9.15, batch 4 7.95 -> 7.37,
-// batch 5 with 121 synapse types 12.84 -> 12.77 (there the scatter is as long as the dense phase).
+// step one row at a time and in pairs, 66,634 neurons at 4 Hz: batch 5 10.00 -> 9.20, batch 4 7.95 -> 7.50,
+// batch 5 with 121 synapse types 12.84 -> 12.72 (there the scatter is as long as the dense phase).
 struct f2 {
   unsigned long long x;
 };
@@ -46,9 +46,12 @@ __device__ __forceinline__ f2 pack2(float lo, float hi) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(d.x) : "f"(lo), "f"(hi));
   return d;
 }
-__device__ __forceinline__ f2 mul(f2 a, f2 b) {
+// The assembler contracts a packed multiply and a packed add even under -fmad=false, which changes the
+// results (a third of the voltages of one step in their last bit).  A product is therefore a multiply-add
+// of a minus zero that the compiler cannot know: a * b + (-0) is a * b, rounded once, sign of zero included.
+__device__ __forceinline__ f2 mul_nz(f2 a, f2 b, unsigned long long minus_zero) {
   f2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.x) : "l"(a.x), "l"(b.x));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.x) : "l"(a.x), "l"(b.x), "l"(minus_zero));
   return d;
 }
 __device__ __forceinline__ f2 add(f2 a, f2 b) {
@@ -61,7 +64,7 @@ __device__ __forceinline__ f2 sub(f2 a, f2 b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d.x) : "l"(a.x), "l"(b.x));
   return d;
 }
-__device__ __forceinline__ float mul(float a, float b) { return a * b; }
+__device__ __forceinline__ float mul_nz(float a, float b, unsigned long long) { return a * b; }
 __device__ __forceinline__ float add(float a, float b) { return a + b; }
 __device__ __forceinline__ float sub(float a, float b) { return a - b; }
 template <int W> __device__ __forceinline__ typename RowVec<W>::T all(float v);
@@ -85,6 +88,7 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int D = a.D, K = a.K, N = a.N, Np = a.Np;
+  auto mul = [&](auto x, auto y) { return mul_nz(x, y, a.minus_zero2); };
   // equal slices, or slices of equal scatter work (at most one neuron per thread either way)
   const int n0 = a.slice ? a.slice[blockIdx.x] : blockIdx.x * a.chunk;
   const int cn = a.slice ? a.slice[blockIdx.x + 1] - n0 : min(a.chunk, N - n0);
@@ -92,7 +96,7 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
   // One thread of the last warp arrives at and waits on the phase counters.  Its release completes only
   // when the block's atomics of the step have been performed, and whatever shares its warp waits with it;
   // the last warp is the one with the fewest neurons (none at up to 480 per block).  5,000 neurons, batch 2:
-  // 5.11 us per step with thread 0, 4.37 with the last warp; no difference at 450 neurons per block.
+  // 5.11 us per step with thread 0, 4.40 with the last warp; no difference at 450 neurons per block.
   const bool ctl = tid == NT - 32;
   const int n = n0 + (active ? tid : 0);
   const int nb = B_ * a.n_bkg;
