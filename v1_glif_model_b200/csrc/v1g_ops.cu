@@ -137,9 +137,22 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const float* __restric
 }
 
 template <int BP>
-struct alignas(BP * 4 > 16 ? 16 : BP * 4) GatherRow {
+struct alignas(BP * 4) GatherRow {
   float v[BP];
 };
+// a whole row in one load: with 32 bytes as two loads every lane pays its own L1 line access twice
+template <int BP>
+__device__ __forceinline__ GatherRow<BP> load_row(const GatherRow<BP>* p) {
+  if constexpr (BP == 8) {
+    GatherRow<8> g;
+    asm volatile("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(g.v[0]), "=f"(g.v[1]), "=f"(g.v[2]), "=f"(g.v[3]), "=f"(g.v[4]), "=f"(g.v[5]), "=f"(g.v[6]), "=f"(g.v[7])
+                 : "l"(p));
+    return g;
+  } else {
+    return *p;
+  }
+}
 
 // LPR lanes walk one row of the CSR, U synapses each at a time with all their loads in flight
 template <int BP, bool PROJ, int LPR>
@@ -181,7 +194,7 @@ __global__ void __launch_bounds__(256) gather_dx_kernel(
         GatherRow<BP> gr[U];
 #pragma unroll
         for (int q = 0; q < U; ++q)
-          if (s[q] >= 0) gr[q] = rw[(int64_t)p[q] * S + s[q]];
+          if (s[q] >= 0) gr[q] = load_row<BP>(rw + (int64_t)p[q] * S + s[q]);
 #pragma unroll
         for (int q = 0; q < U; ++q)
           if (s[q] >= 0) {
@@ -194,7 +207,7 @@ __global__ void __launch_bounds__(256) gather_dx_kernel(
           if (s[q] < 0) continue;
           for (int r = 0; r < R; ++r) {
             const float wb = wv[q] * basis_s[s[q] * R + r];
-            const GatherRow<BP> gr = rw[(int64_t)p[q] * R + r];
+            const GatherRow<BP> gr = load_row<BP>(rw + (int64_t)p[q] * R + r);
 #pragma unroll
             for (int b = 0; b < BP; ++b) acc[b] += gr.v[b] * wb;
           }
