@@ -539,7 +539,8 @@ class V1Column:
     def _rollout_wide(self, x, bkg_counts, state, z, v, save_for_bwd):
         """Forward rollout of more trials than one kernel launch takes (``V1G_MAX_BATCH``; the reference
         evaluates 10 trials per angle, ``osi_dsi_estimator.py:424``): trials are independent, so the
-        batch runs as consecutive groups of at most 8, each on its rows of the inputs, outputs and state.
+        batch runs as consecutive groups of at most 8 and about equal size, each on its rows of the inputs,
+        outputs and state.
         Counts that the library is to draw are drawn for the whole batch first, so that row ``i`` gets the
         noise of batch row ``i`` and not that of its position inside a group."""
         if save_for_bwd:
@@ -550,8 +551,11 @@ class V1Column:
             if state is not None and len(state) > 6 and isinstance(state[6], torch.Tensor):
                 first = int(state[6][0])
             bkg_counts = self.sample_bkg_counts(b, t_len, first_step=first)
-        for lo in range(0, b, _lib.MAX_BATCH):
-            hi = min(b, lo + _lib.MAX_BATCH)
+        # groups of about equal size: the widest kernels (7 and 8 trials) take the most time per trial, 8 trials
+        # 16.5 us per step at 66,634 neurons against 9.2 for 5
+        groups = -(-b // _lib.MAX_BATCH)
+        bounds = [b * g // groups for g in range(groups + 1)]
+        for lo, hi in zip(bounds[:-1], bounds[1:]):
             sub = tuple(s[lo:hi] for s in state) if state is not None else None
             st = C.byref(self._state_struct(sub)) if sub is not None else None
             self._check(self._lib.v1g_rollout_fwd(
