@@ -9,13 +9,14 @@ import torch
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("batch", [1, 2, 3, 5, 6, 7, 8])
+@pytest.mark.parametrize("batch,n_bkg", [(1, 20), (2, 20), (3, 20), (5, 20), (6, 20), (7, 20), (8, 20),
+                                         (6, 200)])      # more counts per step than 2 per thread
 @pytest.mark.parametrize("n_receptors", [4, 5])
-def test_paired_rows_round_like_single_rows(batch, n_receptors):
+def test_paired_rows_round_like_single_rows(batch, n_bkg, n_receptors):
     from util import make_case, make_inputs
     from v1_glif_model_b200 import synth
     from v1_glif_model_b200.models import V1Column
-    cfg, dicts, _ = make_case(dataclasses.replace(synth.CONFIGS["small"], batch=batch, n_receptors=n_receptors))
+    cfg, dicts, _ = make_case(dataclasses.replace(synth.CONFIGS["small"], batch=batch, n_bkg=n_bkg, n_receptors=n_receptors))
     cell = V1Column(*dicts)
     x, c = (torch.from_numpy(t).cuda() for t in make_inputs(cfg, seq_len=40))
     out = []

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256) scatter_dw_kernel(
 // {1, 2, 4, 8} floats (32 bytes at most).  With few synapse types (PROJ) the basis is applied there too
 // and a synapse reads one such row, its type's; otherwise it reads the R rows of its target.  Currents and
 // both gradients of one step at 66,634 neurons, batch 5 (8 M synapses): 536 us with a pass over the
-// synapses per batch row, 157 us with this.
+// synapses per batch row, 145 us with this.
 constexpr int PROJ_MAX_TYPES = 8;
 
 template <int BP, bool PROJ>

@@ -23,7 +23,11 @@
 
 namespace {
 
-constexpr int NT = 768;
+// 512 threads leave 128 registers, room for one entry in flight ahead of the one at work.  230,924 neurons,
+// batch 4, us per step: 768 threads without it 82.4, with the packed rows of the scatter phase 72.8, 512
+// threads with both 69.8; 100,000 neurons, batch 8, dense basis 64.0 / 61.8 / 60.4.
+constexpr int NT = 512;
+constexpr int COUNTS = 3;  // background counts a thread fetches per step: batch * n_bkg <= COUNTS * NT
 
 // bit d-1 of hist0[b*N+n] = neuron n of batch row b spiked d steps before the rollout starts
 // LGN event list with the bounds of each event's synapse row, so that the rollout kernels need no
@@ -261,10 +265,10 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_kernel(const FwdArgs a) {
     const int slot = consume ? (t - 2) % K : 0;
     const int* cnt_s = s_cnt + (t & 1) * nb;  // counts of step t-2
     // prefetch the counts of step t-1 (used by iteration t+1)
-    int cnt_next[2] = {0, 0};
+    int cnt_next[COUNTS] = {};
     if (t >= 1 && t + 1 < a.T + 2) {
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < COUNTS; ++q) {
         const int i = tid + q * NT;
         if (i < nb) {
           const int b = i / a.n_bkg, j = i - b * a.n_bkg;
@@ -277,36 +281,52 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_kernel(const FwdArgs a) {
     int* nspk_p = &s_misc[2 + (t & 1)];
 
     // ---------------- dense phase ----------------
+    // The whole state of an entry is read before the previous entry is written back: a load may not pass
+    // an earlier store to the same array, and when the state lives in a global slab every read that had to
+    // wait for the stores before it cost an L2 round trip of its own.
     float I[R_], In[R_];
+    struct Entry {
+      unsigned hist, r;
+      float v, a0, a1, pr[R_], p[R_];
+    } cur, nxt;
+    auto load_entry = [&](int b, int k, Entry& e) {
+      const int si = b * chunkP + k;
+      e.hist = S_hist[si];
+      e.r = S_r[si];
+      e.v = S_v[si];
+      e.a0 = S_a0[si];
+      e.a1 = S_a1[si];
+#pragma unroll
+      for (int r = 0; r < R_; ++r) {
+        e.pr[r] = S_pr[(r * B + b) * chunkP + k];
+        e.p[r] = S_p[(r * B + b) * chunkP + k];
+      }
+    };
     int b = 0, k = tid;
     while (k >= cn && b < B) { k -= cn; ++b; }
-    if (consume && b < B) load_ring(b, k, slot, I);
+    if (b < B) {
+      if (consume) load_ring(b, k, slot, I);
+      load_entry(b, k, cur);
+    }
     while (b < B) {
       int bn = b, kn = k + NT;
       while (kn >= cn && bn < B) { kn -= cn; ++bn; }
-      if (consume && bn < B) load_ring(bn, kn, slot, In);
+      if (bn < B) {
+        if (consume) load_ring(bn, kn, slot, In);
+        load_entry(bn, kn, nxt);
+      }
       const int n = n0 + k;
       const int si = b * chunkP + k;
       if (consume) finish_input(b, k, slot, cnt_s, I);
-      // The whole state of the entry is read before any of it is written back: a load may not pass
-      // an earlier store to the same array, and when the state lives in a global slab every read that
-      // had to wait for the stores before it cost an L2 round trip of its own.
-      const unsigned hist = S_hist[si];
-      float pr_in[R_], p_in[R_];
-#pragma unroll
-      for (int r = 0; r < R_; ++r) {
-        pr_in[r] = S_pr[(r * B + b) * chunkP + k];
-        p_in[r] = S_p[(r * B + b) * chunkP + k];
-      }
-      const float a0 = S_a0[si], a1 = S_a1[si];
-      const float v = S_v[si];
-      const int r_in = (int)S_r[si];
+      const unsigned hist = cur.hist;
+      const float a0 = cur.a0, a1 = cur.a1, v = cur.v;
+      const int r_in = (int)cur.r;
       const float prev_z = (hist & 1u) ? 1.f : 0.f;
       float csum = 0.f;
 #pragma unroll
       for (int r = 0; r < R_; ++r) {
         const int pi = (r * B + b) * chunkP + k;
-        float pr = pr_in[r], p = p_in[r];
+        float pr = cur.pr[r], p = cur.p[r];
         if (consume) {
           pr = pr * a.sd[r] + I[r] * a.pinit[r];  // psc_rise(t-2)
           S_pr[pi] = pr;
@@ -339,13 +359,14 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_kernel(const FwdArgs a) {
       if (z) spk_list[atomicAdd(nspk_p, 1)] = ((uint32_t)b << 24) | (uint32_t)k;
 #pragma unroll
       for (int r = 0; r < R_; ++r) I[r] = In[r];
+      cur = nxt;
       b = bn;
       k = kn;
     }
     {
       int* cnt_n = s_cnt + ((t + 1) & 1) * nb;
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
+      for (int q = 0; q < COUNTS; ++q) {
         const int ii = tid + q * NT;
         if (ii < nb) cnt_n[ii] = cnt_next[q];
       }
@@ -359,16 +380,50 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_kernel(const FwdArgs a) {
       s_misc[2 + ((t + 1) & 1)] = 0;
     }
     const int nspk = *nspk_p;
-    for (int e = warp; e < nspk; e += NW) {
-      const uint32_t ent = spk_list[e];
-      if (a.stat_neuron && lane == 0) {
-        atomicAdd(a.stat_neuron + n0 + (int)(ent & 0xffffff), 1);
-        atomicAdd(a.stat_pop + t * B + (int)(ent >> 24), 1);
+    // every lane fetches the row bounds of one of the warp's next 32 spikes
+    for (int e0 = warp; e0 < nspk; e0 += 32 * NW) {
+      const int e = e0 + lane * NW;
+      uint32_t ent = 0;
+      int j0 = 0, j1 = 0;
+      if (e < nspk) {
+        ent = spk_list[e];
+        const int n = n0 + (int)(ent & 0xffffff);
+        if (a.stat_neuron) {
+          atomicAdd(a.stat_neuron + n, 1);
+          atomicAdd(a.stat_pop + t * B + (int)(ent >> 24), 1);
+        }
+        if (a.rec_syn8) {
+          j0 = a.rec_rowptr[(int64_t)n * D];
+          j1 = a.rec_rowptr[(int64_t)n * D + D];
+          c_rec_ev += (unsigned long long)(j1 - j0);
+        }
       }
-      walk_rec((int)(ent >> 24), n0 + (int)(ent & 0xffffff), t);
+      const int m = min(32, (nspk - e0 + NW - 1) / NW);
+      for (int i = 0; i < m; ++i) {
+        const uint32_t en = __shfl_sync(0xffffffffu, ent, i);
+        const int r0 = __shfl_sync(0xffffffffu, j0, i), r1 = __shfl_sync(0xffffffffu, j1, i);
+        if (a.rec_syn8)
+          v1g_scatter_row8<R_>(a, a.rec_syn8, basis_s, lane, (int)(en >> 24), r0, r1, t % K, true);
+        else
+          walk_rec((int)(en >> 24), n0 + (int)(en & 0xffffff), t);
+      }
     }
     if (tid == 0) c_spikes += (unsigned long long)nspk;
-    if (t + 1 < a.T) scatter_lgn(t + 1);
+    if (t + 1 < a.T) {
+      if (a.lgn_syn8) {
+        const int e1 = v1g_lgn_begin(a, t + 2);
+        for (int e = v1g_lgn_begin(a, t + 1) + (NW - 1 - warp) * gridDim.x + blockIdx.x; e < e1; e += gridDim.x * NW) {
+          const uint4 ent = a.lgn_ent4[e];
+          v1g_scatter_row8<R_>(a, a.lgn_syn8, basis_s, lane, (int)(ent.x >> 24), (int)ent.y, (int)ent.z, (t + 1) % K, false);
+          if (lane == 0) {
+            c_lgn_rows += 1;
+            c_lgn_ev += (unsigned long long)(ent.z - ent.y);
+          }
+        }
+      } else {
+        scatter_lgn(t + 1);
+      }
+    }
     if (prof) {
       const unsigned long long ph3 = gtime();
       ph_barrier += ph1 - ph0;
@@ -646,7 +701,7 @@ static int rollout_fwd_impl(V1GHandle* h, int32_t batch, int32_t n_steps, const 
   const V1GSource& ls = h->src[V1G_SRC_LGN];
   a.rec_rowptr = rs.rowptr; a.rec_post = rs.post; a.rec_w = rs.w; a.rec_sid = rs.sid;
   a.lgn_rowptr = ls.rowptr; a.lgn_post = ls.post; a.lgn_w = ls.w; a.lgn_sid = ls.sid;
-  a.bkg_inptr = bk.in_ptr; a.bkg_inpre = bk.in_pre; a.bkg_w = bk.gather_w(); a.bkg_insid = bk.in_sid;
+  a.bkg_rowptr = bk.rowptr; a.bkg_inptr = bk.in_ptr; a.bkg_inpre = bk.in_pre; a.bkg_w = bk.gather_w(); a.bkg_insid = bk.in_sid;
   a.decay = h->decay; a.cf = h->cf; a.asc_decay = h->asc_decay; a.asc_amps = h->asc_amps;
   a.basis = h->basis; a.tref = h->tref;
   for (int r = 0; r < V1G_MAX_RECEPTORS; ++r) {
@@ -676,8 +731,8 @@ static int rollout_fwd_impl(V1GHandle* h, int32_t batch, int32_t n_steps, const 
     a.phase_ns = h->phase_ns;
     h->phase_grid = plan.grid;
   }
-  if (2 * NT < B * c.n_bkg)
-    return v1g_fail(h, V1G_ERANGE, "batch*n_bkg=%d exceeds %d", B * c.n_bkg, 2 * NT);
+  if (COUNTS * NT < B * c.n_bkg)
+    return v1g_fail(h, V1G_ERANGE, "batch*n_bkg=%d exceeds %d", B * c.n_bkg, COUNTS * NT);
 
   // Register-resident kernel when the slice fits one neuron per thread and the (R, B) pair is
   // instantiated; the shared-memory kernel otherwise.

@@ -13,7 +13,7 @@ struct FwdArgs {
   const int32_t *lgn_rowptr, *lgn_post;
   const float* lgn_w;
   const uint8_t* lgn_sid;
-  const int32_t *bkg_inptr, *bkg_inpre;
+  const int32_t *bkg_inptr, *bkg_inpre, *bkg_rowptr;
   const float* bkg_w;
   const uint8_t* bkg_insid;
   // neuron constants

@@ -6,6 +6,7 @@
 // Used when the block slice has at most V1G_NT_REG neurons; otherwise the shared-memory kernel in
 // v1g_rollout_fwd.cu runs.  Synchronisation, ring protocol and arithmetic (operation order
 // included) are identical to that kernel.
+#include <algorithm>
 #include <type_traits>
 
 #include "v1g_rollout_fwd.cuh"
@@ -190,7 +191,6 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
 
   // event counters of the warp's lane 0 (in shared memory: the registers are all taken)
   unsigned long long *ctr = ctr_s + 4 * warp, &c_rec_ev = ctr[0], &c_lgn_rows = ctr[1], &c_lgn_ev = ctr[2], &c_spikes = ctr[3];
-  unsigned c_bkg_rows = 0;
   // LGN events are dealt out over the grid's warps block by block (event i to block i mod grid), the
   // last warps of a block first: numbered block-major, the few hundred events of a step all fell on
   // the first third of the blocks, which then set the pace of every step
@@ -238,12 +238,11 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
   const bool prof = a.phase_ns != nullptr && tid == 0;
   unsigned long long *ph = ctr_s + 4 * NW, &ph_dense = ph[0], &ph_scatter = ph[1], &ph_barrier = ph[2];
   if (prof) ph[3] = gtime();
-  unsigned long long seen = 0;
+  bool seen = false;   // the phase that the next iteration waits for is complete (thread ctl)
   bool ok = true;
 
   // background input of W batch rows of this neuron: sum over its in-synapses of
   // (w * count) * basis[sid, :] (models.py:890-934 in post-major form)
-  unsigned c_bkg32 = 0;  // delivered background events of this thread (widened at the end)
   auto bkg_gather = [&](auto wc_, int b, const int* cnt_s, auto& Gs) {
     constexpr int W = decltype(wc_)::value;
 #pragma unroll
@@ -262,14 +261,12 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
           Gs[r] = add(Gs[r], mul(wc, f2{q.x}));
           if (r + 1 < R_) Gs[r + 1] = add(Gs[r + 1], mul(wc, f2{q.y}));
         }
-        c_bkg32 += (cnt.x > 0 ? 1u : 0u) + (cnt.y > 0 ? 1u : 0u);
       } else {
         const int cnt = *cp;
         const float wc = __uint_as_float(e.y) * (float)cnt;
         const float* bs = basis_s + (e.x >> 24) * R_;
 #pragma unroll
         for (int r = 0; r < R_; ++r) Gs[r] += wc * bs[r];
-        c_bkg32 += cnt > 0 ? 1u : 0u;
       }
     }
   };
@@ -280,9 +277,8 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
     const unsigned long long ph0 = prof ? gtime() : 0;
     if (ctl && t >= 2) {
       const unsigned long long target = v1g_phase_target(t - 2, G);
-      if (seen < target)
-        seen = v1g_wait(v1g_phase_counter(a.barrier, t - 2), target, a.spin_limit, a.status);
-      if (seen < target) s_misc[1] = 1;
+      if (!seen) seen = v1g_wait(v1g_phase_counter(a.barrier, t - 2), target, a.spin_limit, a.status) >= target;
+      if (!seen) s_misc[1] = 1;
     }
     __syncthreads();
     if (s_misc[1]) {
@@ -297,17 +293,11 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
     if (t >= 1) {
       // counts of step t-1 for the next iteration, copied asynchronously into the other buffer
       int* cnt_n = s_cnt + ((t + 1) & 1) * BP * a.n_bkg;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int i = tid + q * NT;
-        if (i < nb) {
-          const int b = i / a.n_bkg, j = i - b * a.n_bkg;
-          cp_async_4(cnt_n + j * BP + b, a.bkg_counts + ((int64_t)b * a.T + (t - 1)) * a.n_bkg + j);
-        }
+      for (int i = tid; i < nb; i += NT) {
+        const int b = i / a.n_bkg, j = i - b * a.n_bkg;
+        cp_async_4(cnt_n + j * BP + b, a.bkg_counts + ((int64_t)b * a.T + (t - 1)) * a.n_bkg + j);
       }
     }
-    if (blockIdx.x == 0 && consume)
-      for (int i = tid; i < BP * a.n_bkg; i += NT) c_bkg_rows += cnt_s[i] > 0 ? 1 : 0;
     int* nspk_p = &s_misc[2 + (t & 1)];
 
 #ifndef V1G_FWD_NO_ROW_PREFETCH
@@ -453,7 +443,7 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
     const unsigned long long ph2 = prof ? gtime() : 0;
     // ---------------- scatter phase ----------------
     if (ctl) {
-      seen = (t >= 1) ? v1g_ld_acquire(v1g_phase_counter(a.barrier, t - 1)) : 0;
+      seen = t >= 1 && v1g_ld_acquire(v1g_phase_counter(a.barrier, t - 1)) >= v1g_phase_target(t - 1, G);
       s_misc[2 + ((t + 1) & 1)] = 0;
     }
     const int nspk = *nspk_p;
@@ -530,8 +520,7 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
     if (ok && a.T >= 1) v1g_arrive(v1g_phase_counter(a.barrier, a.T));
     const unsigned long long target = v1g_phase_target(a.T, G);
     if (ok) {
-      seen = v1g_wait(v1g_phase_counter(a.barrier, a.T), target, a.spin_limit, a.status);
-      if (seen < target) s_misc[1] = 1;
+      if (v1g_wait(v1g_phase_counter(a.barrier, a.T), target, a.spin_limit, a.status) < target) s_misc[1] = 1;
     }
   }
   __syncthreads();
@@ -544,8 +533,6 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
         s_cnt[j * BP + b] = a.bkg_counts[((int64_t)b * a.T + s) * a.n_bkg + j];
       }
       __syncthreads();
-      if (blockIdx.x == 0)
-        for (int i = tid; i < BP * a.n_bkg; i += NT) c_bkg_rows += s_cnt[i] > 0 ? 1 : 0;
       if (active) {
         float* rp = a.ring + ((int64_t)(s % K) * B_ * R_) * Np + n;
 #pragma unroll
@@ -587,19 +574,37 @@ __global__ void __launch_bounds__(NT, 1) rollout_fwd_reg_kernel(const FwdArgs a)
       for (int d = 0; d < D; ++d) a.st.z_buf[((int64_t)b * D + d) * N + n] = (rh[b] >> d) & 1u ? 1.f : 0.f;
     }
   }
-  const unsigned long long s_bkg_ev = v1g_warp_sum((unsigned long long)c_bkg32);
-  const unsigned long long s_bkg_rows = v1g_warp_sum((unsigned long long)c_bkg_rows);
   if (lane == 0) {
     V1GCounters* c = (V1GCounters*)a.counters;
     if (c_rec_ev) atomicAdd(&c->rec_events, c_rec_ev);
     if (c_lgn_rows) atomicAdd(&c->lgn_rows, c_lgn_rows);
     if (c_lgn_ev) atomicAdd(&c->lgn_events, c_lgn_ev);
-    if (s_bkg_ev) atomicAdd(&c->bkg_events, s_bkg_ev);
-    if (s_bkg_rows) atomicAdd(&c->bkg_rows, s_bkg_rows);
     if (tid == 0 && c_spikes) {
       atomicAdd(&c->spikes, c_spikes);
       atomicAdd(&c->rec_rows, c_spikes * (unsigned long long)D);
     }
+  }
+}
+
+// Background rows and events of a rollout: every synapse of a node with a count is delivered once, whatever
+// the block.  Counted here and not where they are delivered: there it took 4 of 26 instructions per
+// synapse and pair of rows.
+__global__ void __launch_bounds__(256) count_bkg_kernel(const int32_t* __restrict__ counts, int64_t total, int n_bkg,
+                                                        const int32_t* __restrict__ rowptr,
+                                                        unsigned long long* __restrict__ counters) {
+  unsigned long long rows = 0, events = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
+    if (counts[i] > 0) {
+      const int j = (int)(i % n_bkg);
+      rows += 1;
+      events += (unsigned long long)(rowptr[j + 1] - rowptr[j]);
+    }
+  rows = v1g_warp_sum(rows);
+  events = v1g_warp_sum(events);
+  if ((threadIdx.x & 31) == 0 && rows) {
+    V1GCounters* c = (V1GCounters*)counters;
+    atomicAdd(&c->bkg_rows, rows);
+    atomicAdd(&c->bkg_events, events);
   }
 }
 
@@ -616,7 +621,11 @@ int launch(V1GHandle* h, const FwdArgs& a, int grid, size_t smem, cudaStream_t s
   V1G_CUDA(h, cudaLaunchCooperativeKernel((void*)kern, dim3(grid), dim3(NT), args, smem, st));
   V1G_CUDA(h, cudaEventRecord(h->ev[1], st));
   h->ev_valid[0] = true;
-  v1g_count_launches(1);
+  const int64_t n_counts = (int64_t)a.B * a.T * a.n_bkg;
+  count_bkg_kernel<<<(unsigned)std::min<int64_t>((n_counts + 1023) / 1024, h->n_sms), 256, 0, st>>>(
+      a.bkg_counts, n_counts, a.n_bkg, a.bkg_rowptr, a.counters);
+  V1G_CUDA(h, cudaGetLastError());
+  v1g_count_launches(2);
   return V1G_OK;
 }
 
